@@ -33,15 +33,25 @@ constexpr uint32_t kCellTable = 4096;  // cells per axis of the plain path's cel
 constexpr uint32_t kErrWatchdogTraverse = 1u;
 constexpr uint32_t kErrWatchdogLight = 2u;
 
+// A node of one threaded ordering.  The rays of ordering o (cube_face) have axis o >> 1 as their major
+// axis and know its sign, so that axis' planes are stored as the near and the far one; the other two
+// axes follow the order x, y, z.  The pairs are operands of the two-lane slab arithmetic (RayX).
 struct __align__(32) NodeX {
-    float bmin[3];
-    int32_t miss;  // position in the same ordering, -1 = end
-    float bmax[3];
-    int32_t tri;   // -1 internal; leaf: triangle id, | kEmitterBit for lights
+    float lo[2], hi[2];  // minor axes: lower and upper planes
+    float near, far;     // major axis
+    int32_t miss;        // position in the same ordering, -1 = end
+    int32_t tri;         // -1 internal; leaf: triangle id, | kEmitterBit for lights
 };
 static_assert(sizeof(NodeX) == 32, "NodeX is one 32-byte sector");
 
-// 32 bytes of read-only data in one 256-bit global load (sm_100 and later); p 32-byte aligned
+// 32 bytes of read-only data as four register pairs in one 256-bit global load (sm_100 and later);
+// p 32-byte aligned
+__device__ __forceinline__ void ldg32q(const void* p, unsigned long long& a, unsigned long long& b,
+                                       unsigned long long& c, unsigned long long& d) {
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p));
+}
+
+// ... and as eight words
 __device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b) {
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
@@ -202,6 +212,14 @@ __device__ __forceinline__ void bin_cost_add(const RayQueue& q, uint32_t bin, ui
     }
 }
 
+// Lanes of each warp that take rays when the launch has fewer rays than lanes: the rays spread over
+// all warps, as lanes of one warp that are at different points of their walks (a node, a triangle)
+// wait for each other's loads.
+__device__ __forceinline__ uint32_t spread_lanes(uint32_t rays) {
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    return (rays + warps - 1) / warps;
+}
+
 // counting-sort photon grid of the jobs of a launch with SPPM_FLAG_PHOTON_GRID, rebuilt every
 // pass: the records of job k's hash slot s are rec[ofs[b + s]] .. rec[ofs[b + s + 1] - 1], b = the
 // job's first hash slot in the launch (the hash-slot launch set's prefix[k]); photon_grid.cuh has
@@ -285,6 +303,66 @@ __device__ __forceinline__ f3 refract(f3 i, f3 n, float eta) {
 }
 __device__ __forceinline__ float signf(float x) { return x > 0.0f ? 1.0f : (x < 0.0f ? -1.0f : 0.0f); }
 __device__ __forceinline__ float fractf(float x) { return xsub(x, floorf(x)); }
+
+// ---- the box test of raytrace() (eyeraytrace.fs:160-176, photontrace.fs:150-166) -------------
+// Two-lane single-precision arithmetic: each lane of add2 and mul2 is the scalar IEEE operation.
+// mul2 is a fused multiply-add of -0, exact for every product: the assembler joins mul.rn.f32x2 with
+// a following add.rn.f32x2 into one fused operation (with contraction off too, and through a literal
+// -0; 45 % of random operands then differ from the scalar pair), which it cannot do with an addend
+// whose value it does not know.
+static __constant__ float2 k_minus_zero2 = {-0.0f, -0.0f};
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(pack2(k_minus_zero2.x, k_minus_zero2.y)));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// a ray's slab operands in the layout of its ordering's nodes: 1/d and -(1/d) * org of the minor axes,
+// and the major axis' twice
+struct RayX {
+    unsigned long long r, o, rm, om;
+};
+__device__ __forceinline__ RayX ray_x(f3 org, f3 dir, int face) {
+    const f3 rcp = mk(xdiv(1.0f, dir.x), xdiv(1.0f, dir.y), xdiv(1.0f, dir.z));
+    const f3 t0 = mul(neg(rcp), org);
+    const int m = face >> 1;
+    RayX R;
+    R.r = pack2(m == 0 ? rcp.y : rcp.x, m == 2 ? rcp.y : rcp.z);
+    R.o = pack2(m == 0 ? t0.y : t0.x, m == 2 ? t0.y : t0.z);
+    const float rm = m == 0 ? rcp.x : (m == 1 ? rcp.y : rcp.z), om = m == 0 ? t0.x : (m == 1 ? t0.y : t0.z);
+    R.rm = pack2(rm, rm);
+    R.om = pack2(om, om);
+    return R;
+}
+// The box's interval along the ray: max over the axes of the nearer plane's distance, min of the
+// farther one's, each fl(fl(plane * r) + o).  ORDERED: no direction component is degenerate, so the
+// major axis' near plane is the nearer one; otherwise it is taken by minimum and maximum like the
+// minor axes (a zero component makes distances NaN, which minimum and maximum drop).
+template <bool ORDERED>
+__device__ __forceinline__ void slab_x(const RayX& R, unsigned long long lo, unsigned long long hi,
+                                       unsigned long long near_far, float& tmin, float& tmax) {
+    float la, lb, ha, hb, n, f;
+    unpack2(add2(mul2(R.r, lo), R.o), la, lb);
+    unpack2(add2(mul2(R.r, hi), R.o), ha, hb);
+    unpack2(add2(mul2(R.rm, near_far), R.om), n, f);
+    tmin = fmax3(fminf(la, ha), fminf(lb, hb), ORDERED ? n : fminf(n, f));
+    tmax = fmin3(fmaxf(la, ha), fmaxf(lb, hb), ORDERED ? f : fmaxf(n, f));
+}
+__device__ __forceinline__ int32_t node_miss(unsigned long long links) { return (int32_t)(uint32_t)links; }
+__device__ __forceinline__ int32_t node_tri(unsigned long long links) { return (int32_t)(links >> 32); }
 
 // ---- the triangle test of raytrace() (eyeraytrace.fs:200-243, photontrace.fs:196-236) --------
 // Moller-Trumbore on the packed operands (a = v0 | e0.x, b = e0.yz | e1.xy, c.x = e1.z), every

@@ -71,9 +71,9 @@ __device__ __forceinline__ Hit trace_exact(const DevScene& s, f3 org, f3 dir, bo
     h.tri = -1;
     h.mat = -1;
     h.bu = h.bv = h.bw = 0.0f;
-    const NodeX* nodes = s.nodes + (size_t)cube_face(dir) * s.num_nodes;
-    const f3 rcp = mk(xdiv(1.0f, dir.x), xdiv(1.0f, dir.y), xdiv(1.0f, dir.z));
-    const f3 t0 = mul(neg(rcp), org);
+    const int face = cube_face(dir);
+    const NodeX* nodes = s.nodes + (size_t)face * s.num_nodes;
+    const RayX R = ray_x(org, dir, face);
     const int32_t nn = (int32_t)s.num_nodes;
     int32_t i = 0;
     for (int32_t steps = 0;; steps++) {
@@ -81,15 +81,13 @@ __device__ __forceinline__ Hit trace_exact(const DevScene& s, f3 org, f3 dir, bo
             err |= kErrWatchdogTraverse;
             break;
         }
-        float4 A, B;
-        ldg32(nodes + i, A, B);
+        unsigned long long lo, hi, near_far, links;
+        ldg32q(nodes + i, lo, hi, near_far, links);
         if (COUNT) cnt->nodes++;
-        const float lx = xadd(xmul(rcp.x, A.x), t0.x), ly = xadd(xmul(rcp.y, A.y), t0.y), lz = xadd(xmul(rcp.z, A.z), t0.z);
-        const float hx = xadd(xmul(rcp.x, B.x), t0.x), hy = xadd(xmul(rcp.y, B.y), t0.y), hz = xadd(xmul(rcp.z, B.z), t0.z);
-        const float tmin = fmax3(fminf(lx, hx), fminf(ly, hy), fminf(lz, hz));
-        const float tmax = fmin3(fmaxf(lx, hx), fmaxf(ly, hy), fmaxf(lz, hz));
+        float tmin, tmax;
+        slab_x<false>(R, lo, hi, near_far, tmin, tmax);
         const bool hit = (tmin <= tmax) && (tmin <= h.t) && (tmax >= 0.0f);
-        const int32_t tri = __float_as_int(B.w);
+        const int32_t tri = node_tri(links);
         if (hit && tri >= 0 && (!PHOTON || !(tri & kEmitterBit))) {
             const int32_t t = tri & kTriMask;
             if (COUNT) cnt->tris++;
@@ -106,7 +104,7 @@ __device__ __forceinline__ Hit trace_exact(const DevScene& s, f3 org, f3 dir, bo
                 h.bw = u;
             }
         }
-        const int32_t next = hit ? i + 1 : __float_as_int(A.w);
+        const int32_t next = hit ? i + 1 : node_miss(links);
         if (next < 0 || next >= nn) break;
         i = next;
     }
@@ -138,9 +136,9 @@ __device__ __forceinline__ Hit coop_trace_exact_from(const DevScene& s, f3 org, 
     constexpr unsigned kFull = 0xFFFFFFFFu;
     const int lane = (int)(threadIdx.x & 31);
     Hit h = h0;
-    const NodeX* nodes = s.nodes + (size_t)cube_face(dir) * s.num_nodes;
-    const f3 rcp = mk(xdiv(1.0f, dir.x), xdiv(1.0f, dir.y), xdiv(1.0f, dir.z));
-    const f3 t0 = mul(neg(rcp), org);
+    const int face = cube_face(dir);
+    const NodeX* nodes = s.nodes + (size_t)face * s.num_nodes;
+    const RayX R = ray_x(org, dir, face);
     const int32_t nn = (int32_t)s.num_nodes;
     int32_t cur = start;
     uint32_t steps = steps0;
@@ -152,15 +150,13 @@ __device__ __forceinline__ Hit coop_trace_exact_from(const DevScene& s, f3 org, 
         float tmin = 0.0f, tt = 0.0f, bu = 0.0f, bv = 0.0f, bw = 0.0f;
         int32_t miss = -1, tri = -1, mat = -1;
         if (j < nn) {
-            float4 A, B;
-            ldg32(nodes + j, A, B);
-            const float lx = xadd(xmul(rcp.x, A.x), t0.x), ly = xadd(xmul(rcp.y, A.y), t0.y), lz = xadd(xmul(rcp.z, A.z), t0.z);
-            const float hx = xadd(xmul(rcp.x, B.x), t0.x), hy = xadd(xmul(rcp.y, B.y), t0.y), hz = xadd(xmul(rcp.z, B.z), t0.z);
-            tmin = fmax3(fminf(lx, hx), fminf(ly, hy), fminf(lz, hz));
-            const float tmax = fmin3(fmaxf(lx, hx), fmaxf(ly, hy), fmaxf(lz, hz));
+            unsigned long long lo, hi, near_far, links;
+            ldg32q(nodes + j, lo, hi, near_far, links);
+            float tmax;
+            slab_x<false>(R, lo, hi, near_far, tmin, tmax);
             box = (tmin <= tmax) && (tmax >= 0.0f);
-            miss = __float_as_int(A.w);
-            const int32_t raw = __float_as_int(B.w);
+            miss = node_miss(links);
+            const int32_t raw = node_tri(links);
             leaf = raw >= 0 && (!PHOTON || !(raw & kEmitterBit));
             if (leaf && box) {
                 tri = raw & kTriMask;
@@ -298,9 +294,9 @@ __device__ __noinline__ Hit block_trace_exact(const DevScene& s, f3 org, f3 dir,
     constexpr unsigned kFull = 0xFFFFFFFFu;
     const int t = (int)threadIdx.x;
     const int lane = t & 31;
-    const NodeX* nodes = s.nodes + (size_t)cube_face(dir) * s.num_nodes;
-    const f3 rcp = mk(xdiv(1.0f, dir.x), xdiv(1.0f, dir.y), xdiv(1.0f, dir.z));
-    const f3 t0 = mul(neg(rcp), org);
+    const int face = cube_face(dir);
+    const NodeX* nodes = s.nodes + (size_t)face * s.num_nodes;
+    const RayX R = ray_x(org, dir, face);
     const int32_t nn = (int32_t)s.num_nodes;
     if (t == 0) {
         sh.h.t = PHOTON ? 1.0e30f : 1.0e20f;
@@ -321,17 +317,14 @@ __device__ __noinline__ Hit block_trace_exact(const DevScene& s, f3 org, f3 dir,
             float tmin = 0.0f, tt = 0.0f, bu = 0.0f, bv = 0.0f, bw = 0.0f;
             int32_t miss = -1, tri = -1, mat = -1;
             if (j < nn) {
-                float4 A, B;
                 // two 16-byte loads: this toolkit's ptxas fails on the 256-bit form in this function
-                A = __ldg(reinterpret_cast<const float4*>(nodes + j));
-                B = __ldg(reinterpret_cast<const float4*>(nodes + j) + 1);
-                const float lx = xadd(xmul(rcp.x, A.x), t0.x), ly = xadd(xmul(rcp.y, A.y), t0.y), lz = xadd(xmul(rcp.z, A.z), t0.z);
-                const float hx = xadd(xmul(rcp.x, B.x), t0.x), hy = xadd(xmul(rcp.y, B.y), t0.y), hz = xadd(xmul(rcp.z, B.z), t0.z);
-                tmin = fmax3(fminf(lx, hx), fminf(ly, hy), fminf(lz, hz));
-                const float tmax = fmin3(fmaxf(lx, hx), fmaxf(ly, hy), fmaxf(lz, hz));
+                const ulonglong2 A = __ldg(reinterpret_cast<const ulonglong2*>(nodes + j));
+                const ulonglong2 B = __ldg(reinterpret_cast<const ulonglong2*>(nodes + j) + 1);
+                float tmax;
+                slab_x<false>(R, A.x, A.y, B.x, tmin, tmax);
                 box = (tmin <= tmax) && (tmax >= 0.0f);
-                miss = __float_as_int(A.w);
-                const int32_t raw = __float_as_int(B.w);
+                miss = node_miss(B.y);
+                const int32_t raw = node_tri(B.y);
                 leaf = raw >= 0 && (!PHOTON || !(raw & kEmitterBit));
                 if (leaf && box) {
                     tri = raw & kTriMask;
@@ -1524,18 +1517,28 @@ __global__ void __launch_bounds__(256) k_ray_bins_scatter(RayQueue q) {
 }
 
 // trace: persistent warps; a lane whose ray finished fetches the next one from the queue, so
-// lanes stay busy while their neighbours walk longer paths (dynamic fetch)
+// lanes stay busy while their neighbours walk longer paths (dynamic fetch).
+// Bound by instruction issue and L1 wavefronts at 13 to 14 active lanes (a quarter of a step's
+// issue slots test a box, a third a triangle for 3 to 4 lanes), on large meshes by the node loads.
+// So a step does as little as it can: the box test in two-lane arithmetic, the major axis without
+// minimum and maximum (slab_x), one comparison each for the walk's end and for a leaf to test, no
+// step counter of its own: 142.5 -> 126.7 us a launch on the Cornell box (2^20 slots), 744 -> 697 on
+// a 1M-triangle mesh (2^21), 610 -> 568 over 16 jobs.  With fewer rays than lanes the longest walk
+// decides, and what its step waits for: spread over the warps, 2^14 rays take 51 us instead of 70,
+// 2^16 63 instead of 74.
 template <bool COUNT>
 __global__ void __launch_bounds__(128, 9) k_trace_photons(LaunchSet ls, RayQueue q) {
     const uint32_t total = q.counters[0];
     const int refill = q.refill_steps ? (int)q.refill_steps : 32;
     const unsigned lane = threadIdx.x & 31;
     const uint32_t kNeed = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu;
-    uint32_t idx = kNeed;
+    // fewer rays than lanes: spread over all warps (spread_lanes)
+    uint32_t idx = lane < spread_lanes(total) ? kNeed : kDone;
     const NodeX* nodes = nullptr;
     const float4* tri_isect = nullptr;
     int32_t nn = 0;
-    f3 org = mk(0, 0, 0), dir = mk(0, 0, 0), rcp = mk(0, 0, 0), t0 = mk(0, 0, 0);
+    f3 org = mk(0, 0, 0), dir = mk(0, 0, 0);
+    RayX R{};
     Hit h;
     int32_t node = 0, steps = 0;
     uint32_t err = 0;
@@ -1585,10 +1588,10 @@ __global__ void __launch_bounds__(128, 9) k_trace_photons(LaunchSet ls, RayQueue
                     org = mk(o.x, o.y, o.z);
                     dir = mk(d.x, d.y, d.z);
                     nn = (int32_t)S.num_nodes;
-                    nodes = S.nodes + (size_t)cube_face(dir) * nn;
+                    const int face = cube_face(dir);
+                    nodes = S.nodes + (size_t)face * nn;
                     tri_isect = S.tri_isect;
-                    rcp = mk(xdiv(1.0f, dir.x), xdiv(1.0f, dir.y), xdiv(1.0f, dir.z));
-                    t0 = mul(neg(rcp), org);
+                    R = ray_x(org, dir, face);
                     h.t = 1.0e30f;
                     h.tri = -1;
                     h.mat = -1;
@@ -1613,8 +1616,9 @@ __global__ void __launch_bounds__(128, 9) k_trace_photons(LaunchSet ls, RayQueue
             const unsigned drained = __ballot_sync(0xFFFFFFFFu, idx == kDone);
             if (drained && act && (uint32_t)__popc(act) <= q.tail_lanes) {
                 if (idx < kDone) {
+                    const int32_t mat = h.tri >= 0 ? __float_as_int(__ldg(&tri_isect[(size_t)h.tri * 3 + 2]).y) : -1;
                     q.hit[idx] = make_float4(__int_as_float(h.tri), h.bu, h.bv, h.bw);
-                    q.tail_state[idx] = make_float4(h.t, __int_as_float(h.mat), __int_as_float(node),
+                    q.tail_state[idx] = make_float4(h.t, __int_as_float(mat), __int_as_float(node),
                                                     __int_as_float(steps));
                     q.tail_list[atomicAdd(&q.counters[4], 1u)] = idx;
                     idx = kDone;
@@ -1624,51 +1628,53 @@ __global__ void __launch_bounds__(128, 9) k_trace_photons(LaunchSet ls, RayQueue
         }
         if (idx >= kDone) continue;
         bool finished = false;
+        int it = 0;
 #pragma unroll 1
-        for (int it = 0; it < refill; it++) {
-            if (steps++ > nn) {
-                err |= kErrWatchdogTraverse;
-                finished = true;
-                break;
-            }
-            float4 A, B;
-            ldg32(nodes + node, A, B);
+        do {
+            unsigned long long lo, hi, near_far, links;
+            ldg32q(nodes + node, lo, hi, near_far, links);
             if (COUNT) tc.nodes++;
-            const float lx = xadd(xmul(rcp.x, A.x), t0.x), ly = xadd(xmul(rcp.y, A.y), t0.y), lz = xadd(xmul(rcp.z, A.z), t0.z);
-            const float hx = xadd(xmul(rcp.x, B.x), t0.x), hy = xadd(xmul(rcp.y, B.y), t0.y), hz = xadd(xmul(rcp.z, B.z), t0.z);
-            const float tmin = fmax3(fminf(lx, hx), fminf(ly, hy), fminf(lz, hz));
-            const float tmax = fmin3(fmaxf(lx, hx), fmaxf(ly, hy), fmaxf(lz, hz));
+            float tmin, tmax;
+            slab_x<true>(R, lo, hi, near_far, tmin, tmax);
             const bool hit = (tmin <= tmax) && (tmin <= h.t) && (tmax >= 0.0f);
-            const int32_t tri = __float_as_int(B.w);
-            if (hit && tri >= 0 && !(tri & kEmitterBit)) {
+            const int32_t tri = node_tri(links);
+            // a leaf that is no emitter's: neither -1 nor the emitter bit
+            if (hit && (uint32_t)tri < (uint32_t)kEmitterBit) {
                 if (COUNT) tc.tris++;
                 const float4 a = __ldg(&tri_isect[(size_t)tri * 3 + 0]);
                 const float4 b = __ldg(&tri_isect[(size_t)tri * 3 + 1]);
                 const float4 c = __ldg(&tri_isect[(size_t)tri * 3 + 2]);
+                // tri_test_exact with the divisions one after the other's test: few lanes get here at a
+                // time (3 to 4 of a warp), and often none needs the next one
                 const f3 v0 = mk(a.x, a.y, a.z), e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, c.x);
                 const f3 pv = cross(dir, e1);
                 const float det = dot(e0, pv);
                 const f3 tv = sub(org, v0);
                 const f3 qv = cross(tv, e0);
                 const float u = xdiv(dot(tv, pv), det);
-                const float v = xdiv(dot(dir, qv), det);
-                const float tt = xdiv(dot(e1, qv), det);
-                const float w = xsub(xsub(1.0f, u), v);
-                if (u >= 0.0f && v >= 0.0f && tt >= 0.0f && w >= 0.0f && tt < h.t) {
-                    h.t = tt;
-                    h.tri = tri;
-                    h.mat = __float_as_int(c.y);
-                    h.bu = v;
-                    h.bv = w;
-                    h.bw = u;
+                if (u >= 0.0f) {
+                    const float v = xdiv(dot(dir, qv), det);
+                    const float w = xsub(xsub(1.0f, u), v);
+                    if (v >= 0.0f && w >= 0.0f) {
+                        const float tt = xdiv(dot(e1, qv), det);
+                        if (tt >= 0.0f && tt < h.t) {
+                            h.t = tt;
+                            h.tri = tri;
+                            h.bu = v;
+                            h.bv = w;
+                            h.bw = u;
+                        }
+                    }
                 }
             }
-            const int32_t next = hit ? node + 1 : __float_as_int(A.w);
-            if (next < 0 || next >= nn) {
-                finished = true;
-                break;
-            }
-            node = next;
+            node = hit ? node + 1 : node_miss(links);
+            it++;
+            finished = (uint32_t)node >= (uint32_t)nn;
+        } while (!finished && it < refill);
+        steps += it;
+        if (!finished && steps > nn) {
+            err |= kErrWatchdogTraverse;
+            finished = true;
         }
         if (finished) {
             q.hit[idx] = make_float4(__int_as_float(h.tri), h.bu, h.bv, h.bw);

@@ -62,7 +62,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_photons4(LaunchSet ls, Ra
     const int refill = q.refill_steps ? (int)q.refill_steps : 8;
     const unsigned lane = threadIdx.x & 31, tid = threadIdx.x;
     const uint32_t kNeed = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu;
-    uint32_t idx = kNeed;
+    // fewer rays than lanes: spread over all warps (spread_lanes)
+    uint32_t idx = lane < spread_lanes(total) ? kNeed : kDone;
     const Node4Dev* nodes = nullptr;
     const float4* tri_isect = nullptr;
     Ray4 R;

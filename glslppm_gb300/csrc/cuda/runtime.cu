@@ -206,12 +206,16 @@ int pack_scene(const sppm_scene* s, Packed& out) {
             const int32_t raw = s->order_miss[(size_t)o * nn + i];
             NodeX& d = out.nodes[(size_t)o * nn + i];
             const float* b = s->node_bounds + (size_t)c * 6;
-            d.bmin[0] = b[0];
-            d.bmin[1] = b[1];
-            d.bmin[2] = b[2];
-            d.bmax[0] = b[3];
-            d.bmax[1] = b[4];
-            d.bmax[2] = b[5];
+            const int m = o >> 1, a0 = m == 0 ? 1 : 0, a1 = m == 2 ? 1 : 2;
+            d.lo[0] = b[a0];
+            d.hi[0] = b[3 + a0];
+            d.lo[1] = b[a1];
+            d.hi[1] = b[3 + a1];
+            // the major axis' planes in the order the ordering's rays meet them
+            const float p0 = b[m] == b[m] ? b[m] : b[3 + m], p1 = b[3 + m] == b[3 + m] ? b[3 + m] : p0;
+            const bool swap = (p0 > p1) != ((o & 1) != 0);
+            d.near = swap ? p1 : p0;
+            d.far = swap ? p0 : p1;
             d.miss = (raw < 0 || (uint32_t)raw >= nn) ? -1 : raw;
             int32_t tri = s->node_triangle[c];
             if (tri >= (int32_t)nt) return fail(SPPM_ERR_ARG, "node %d: triangle %d out of range", c, tri);
