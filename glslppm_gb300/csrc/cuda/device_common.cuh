@@ -242,7 +242,15 @@ struct LaunchSet {
     uint32_t njobs;
     uint32_t total;
     uint32_t first;
+    uint32_t only;  // job_ids[0]: a launch over one job starts without waiting for the tables
 };
+// job k of a launch and its first item
+__device__ __forceinline__ const JobDesc& job_of(const LaunchSet& ls, int k) {
+    return ls.jobs[ls.njobs == 1 ? ls.only : __ldg(&ls.job_ids[k])];
+}
+__device__ __forceinline__ uint32_t first_item(const LaunchSet& ls, int k) {
+    return ls.njobs == 1 ? 0u : __ldg(&ls.prefix[k]);
+}
 
 __device__ __forceinline__ int find_job(const LaunchSet& ls, uint32_t g) {
     int lo = 0, hi = (int)ls.njobs - 1;

@@ -67,6 +67,7 @@ void launch_resolve_mixed(const LaunchSet& ls, uint32_t display, cudaStream_t s)
 // scan of the slots' counts + the scatter of the records, after the photon pass's last store
 uint32_t grid_tiles(uint32_t hash_slots);
 void launch_grid_sort(const LaunchSet& hash_slots, const LaunchSet& photons, const PhotonGrid& grid, cudaStream_t s);
+// ls covers the pixels in 8x4 tiles (a warp per tile)
 void launch_gather_fp32(const LaunchSet& ls, uint32_t block, cudaStream_t s);
 void launch_resolve_fp32(const LaunchSet& ls, uint32_t display, cudaStream_t s);
 void launch_hash_build(const float4* pos, const float4* flux, uint32_t pw, uint32_t ph, uint32_t hash_num,

@@ -21,8 +21,8 @@ namespace {
 __device__ __forceinline__ uint32_t grid_slot_count(const LaunchSet& hs, uint32_t g) {
     if (g >= hs.total) return 0u;
     const int k = find_job(hs, g);
-    const JobDesc& J = hs.jobs[hs.job_ids[k]];
-    return J.count[g - hs.prefix[k]];
+    const JobDesc& J = job_of(hs, k);
+    return J.count[g - first_item(hs, k)];
 }
 
 // exclusive scan of one value per thread of a kGridScanBlock-thread block; *total = the block's sum
@@ -127,9 +127,9 @@ __global__ void __launch_bounds__(256) k_grid_scatter(LaunchSet ph, const uint32
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ph.total) return;
     const int k = find_job(ph, g);
-    const JobDesc& J = ph.jobs[ph.job_ids[k]];
+    const JobDesc& J = job_of(ph, k);
     if (!(J.flags & SPPM_FLAG_PHOTON_GRID)) return;
-    const uint32_t sidx = g - ph.prefix[k];
+    const uint32_t sidx = g - first_item(ph, k);
     const float4 f = J.ph.flux[sidx];
     if (f.x < 0.0f) return;  // the store's test (photon_store)
     const JobState* st = J.state;

@@ -35,7 +35,7 @@ constexpr int kLocalStack = kStack - kSmemStack;  // deeper entries, in local me
 // at an equal t: does the exact walk meet triangle a before triangle b?  (the leaf ranks of the
 // ray's ordering; looked up only at ties, so the walk keeps no pointer to them)
 __device__ __noinline__ bool met_first(const LaunchSet& ls, int job_k, const Ray4& R, int32_t a, int32_t b) {
-    const DevScene& S = ls.jobs[ls.job_ids[job_k]].scene;
+    const DevScene& S = job_of(ls, job_k).scene;
     if (!S.tri_rank) return false;
     const int32_t* rank = S.tri_rank + (size_t)cube_face(mk(R.dx, R.dy, R.dz)) * S.num_tris;
     return __ldg(&rank[a]) < __ldg(&rank[b]);
@@ -90,11 +90,11 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_photons4(LaunchSet ls, Ra
                     const float4 o = q.org[idx], d = q.dir[idx];
                     const int nk = find_job(ls, __float_as_uint(o.w));
                     if (err && nk != job_k) {  // an error belongs to the job whose ray raised it
-                        atomicOr(&ls.jobs[ls.job_ids[job_k]].state->err, err);
+                        atomicOr(&job_of(ls, job_k).state->err, err);
                         err = 0;
                     }
                     job_k = nk;
-                    const DevScene& S = ls.jobs[ls.job_ids[job_k]].scene;
+                    const DevScene& S = job_of(ls, job_k).scene;
                     nodes = S.nodes4;
                     tri_isect = S.tri_isect;
                     ray4_setup(R, o.x, o.y, o.z, d.x, d.y, d.z);
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_photons4(LaunchSet ls, Ra
             idx = kNeed;
         }
     }
-    if (err) atomicOr(&ls.jobs[ls.job_ids[job_k]].state->err, err);
+    if (err) atomicOr(&job_of(ls, job_k).state->err, err);
 }
 
 // each occupied slot's 32-byte record from its winner (after every photon of the pass is hashed,
@@ -212,8 +212,8 @@ __global__ void __launch_bounds__(256) k_slot_fill(LaunchSet ls) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ls.total) return;
     const int k = find_job(ls, g);
-    const JobDesc& J = ls.jobs[ls.job_ids[k]];
-    const uint32_t slot = g - ls.prefix[k];
+    const JobDesc& J = job_of(ls, k);
+    const uint32_t slot = g - first_item(ls, k);
     uint32_t sidx = J.winner[slot];
     if (sidx == kEmptySlot) return;
     if (sidx == J.PW * J.PH) sidx = 0;  // every photon of the slot clipped: the cleared texel's photon 0
@@ -381,7 +381,7 @@ __device__ __forceinline__ void grid_gather_warp(const LaunchSet& ls, const uint
     const JobState* st = nullptr;
     if (live) {
         k = k_in;
-        const JobDesc& J = ls.jobs[ls.job_ids[k]];
+        const JobDesc& J = job_of(ls, k);
         if ((J.flags & SPPM_FLAG_PHOTON_GRID) && J.px.tri[p] >= 0) {
             st = J.state;
             const bool f64 = (J.flags & SPPM_FLAG_FP64_STATISTICS) != 0;
@@ -435,13 +435,13 @@ __device__ __forceinline__ void grid_gather_warp(const LaunchSet& ls, const uint
     const unsigned long long ucells = (unsigned long long)UX * UY * UZ;
     if (kmin != kmax || ucells > 4ull * own_max || ucells > kCoopMaxCells) {
         if (has) {
-            const JobDesc& J = ls.jobs[ls.job_ids[k]];
+            const JobDesc& J = job_of(ls, k);
             grid_accumulate(grid, __ldg(&slot_prefix[k]), J.hash_num, st, gx, gy, gz, R2f, qn4, fx, fy, fz, M);
         }
         return;
     }
     // the warp's job (uniform)
-    const JobDesc& J = ls.jobs[ls.job_ids[kmin]];
+    const JobDesc& J = job_of(ls, kmin);
     const uint32_t slot_base = __ldg(&slot_prefix[kmin]), hash_num = J.hash_num, nc = (uint32_t)ucells;
     const int Fw = __shfl_sync(full, Fc, __ffs(hasmask) - 1);
     // a lane per cell (rounds of 32 cells): the record ranges, concatenated by a scan; the cells
@@ -549,10 +549,10 @@ __global__ void __launch_bounds__(256) k_gather_mixed(LaunchSet ls, const uint32
     uint32_t p = 0;
     if (live) {
         k = find_job(ls, gi);
-        p = gi - ls.prefix[k];
+        p = gi - first_item(ls, k);
         if (ANY_GRID) {
             // the launch covers each job in 8x4-pixel tiles, a warp per tile (neighbouring hit points)
-            const JobDesc& Jt = ls.jobs[ls.job_ids[k]];
+            const JobDesc& Jt = job_of(ls, k);
             const uint32_t tw = (Jt.W + 7u) >> 3, tile = p >> 5, lane = p & 31u;
             const uint32_t px = (tile % tw) * 8u + (lane & 7u), py = (tile / tw) * 4u + (lane >> 3);
             live = px < Jt.W && py < Jt.H;
@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(256) k_gather_mixed(LaunchSet ls, const uint32
         grid_gather_warp(ls, slot_prefix, grid, live, (uint32_t)k, p, s_grid[threadIdx.x >> 5], gfx, gfy, gfz, gM);
     }
     if (!live) return;
-    const JobDesc& J = ls.jobs[ls.job_ids[k]];
+    const JobDesc& J = job_of(ls, k);
     JobState* st = J.state;
     const uint32_t frame = st->frame;
     if (p == 0) {
@@ -684,8 +684,8 @@ __global__ void k_resolve_mixed(LaunchSet ls, uint32_t display) {
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     if (gi >= ls.total) return;
     const int k = find_job(ls, gi);
-    const JobDesc& J = ls.jobs[ls.job_ids[k]];
-    const uint32_t p = gi - ls.prefix[k];
+    const JobDesc& J = job_of(ls, k);
+    const uint32_t p = gi - first_item(ls, k);
     const bool f64 = (J.flags & SPPM_FLAG_FP64_STATISTICS) != 0;
     const float2 r2 = J.px.stat_r2[p];
     const float r2f = f64 ? (float)reinterpret_cast<const double*>(J.px.stat_r2)[p] : r2.x + r2.y;

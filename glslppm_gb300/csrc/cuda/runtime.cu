@@ -829,6 +829,7 @@ LaunchSet Job::self_set(const JobDesc* table, uint32_t which) const {
     ls.job_ids = d_self;
     ls.prefix = d_self + 1 + 2 * which;
     ls.njobs = 1;
+    ls.only = slot;
     ls.total = which == 0 ? npix : (which == 1 ? P : hash_num);
     return ls;
 }
@@ -959,6 +960,7 @@ int Runner::rebuild() {
         ls.job_ids = d_t + ids;
         ls.prefix = d_t + prefix;
         ls.njobs = nj;
+        ls.only = nj ? t[ids] : 0u;
         ls.total = (uint32_t)total;
         return ls;
     };
@@ -1173,7 +1175,7 @@ int Runner::enqueue_frame(uint32_t phase) {
     if (mixed)
         launch_gather_mixed(any_grid ? pix_tiles : pix, tune.gather_block, fp64_stats, hsh.prefix,
                             any_grid ? &grid : nullptr, stream);
-    else launch_gather_fp32(pix, tune.gather_block, stream);
+    else launch_gather_fp32(pix_tiles, tune.gather_block, stream);
     timed(SPPM_STAGE_GATHER, false);
     return launch_check("SPPM frame");
 }
