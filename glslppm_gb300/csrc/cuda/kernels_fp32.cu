@@ -605,7 +605,7 @@ __global__ void k_frame_begin(LaunchSet ls, RayQueue q) {
         q.counters[4] = 0;
         q.counters[7] += 1u;  // frames since the bins were last reordered
     }
-    if (q.bins && g < kRayBins) q.bins[g] = 0u;
+    if (q.bins && g < kBinCounters * kRayBins) q.bins[g] = 0u;
     if (g >= ls.total) return;
     const int k = find_job(ls, g);
     const JobDesc& J = job_of(ls, k);
@@ -644,7 +644,7 @@ __global__ void k_queue_reset(RayQueue q) {
         q.counters[2] = 0;
         q.counters[4] = 0;
     }
-    if (q.bins && g < kRayBins) q.bins[g] = 0u;
+    if (q.bins && g < kBinCounters * kRayBins) q.bins[g] = 0u;
 }
 
 // ----------------------------------------------------------------------------------------------
@@ -1376,26 +1376,30 @@ __global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
             const unsigned same = __match_any_sync(live, bin);
             const int lead = __ffs(same) - 1;
             uint32_t rb = 0;
-            if ((int)(threadIdx.x & 31) == lead) rb = atomicAdd(&q.bins[bin], __popc(same));
+            const uint32_t counter = blockIdx.x % kBinCounters;
+            if ((int)(threadIdx.x & 31) == lead) rb = atomicAdd(&q.bins[counter * kRayBins + bin], __popc(same));
             rb = __shfl_sync(same, rb, lead);
-            q.key[qi] = make_uint2(bin, rb + __popc(same & ((1u << (threadIdx.x & 31)) - 1)));
+            q.key[qi] = make_uint2(bin | counter << 16, rb + __popc(same & ((1u << (threadIdx.x & 31)) - 1)));
         }
     }
     photon_counters(st, k, active, R.emitted, R.cont ? 1u : 0u, err);
 }
 
-// exclusive scan of the bin counts in place (one block of 1024 threads, 96 bins per thread)
+// exclusive scan of the bin counts in place, a bin's counters one after the other (one block of 1024
+// threads, 12 bins per thread)
 __global__ void __launch_bounds__(1024) k_ray_bins_scan(uint32_t* bins) {
     constexpr uint32_t kPer = kRayBins / 1024;
     static_assert(kRayBins % 1024 == 0 && kPer % 4 == 0, "bin count must split into uint4 chunks");
     __shared__ uint32_t warp_sums[32];
-    uint4* v = reinterpret_cast<uint4*>(bins) + threadIdx.x * (kPer / 4);
+    uint4 v[kBinCounters][kPer / 4];
     uint32_t sum = 0;
-#pragma unroll 4
-    for (uint32_t i = 0; i < kPer / 4; i++) {
-        const uint4 x = v[i];
-        sum += x.x + x.y + x.z + x.w;
-    }
+#pragma unroll
+    for (uint32_t c = 0; c < kBinCounters; c++)
+#pragma unroll
+        for (uint32_t i = 0; i < kPer / 4; i++) {
+            v[c][i] = reinterpret_cast<const uint4*>(bins + c * kRayBins)[threadIdx.x * (kPer / 4) + i];
+            sum += v[c][i].x + v[c][i].y + v[c][i].z + v[c][i].w;
+        }
     const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t incl = sum;
 #pragma unroll
@@ -1416,17 +1420,27 @@ __global__ void __launch_bounds__(1024) k_ray_bins_scan(uint32_t* bins) {
     }
     __syncthreads();
     uint32_t run = warp_sums[warp] + incl - sum;
-#pragma unroll 4
+    auto take = [&](uint32_t& x) {
+        const uint32_t n = x;
+        x = run;
+        run += n;
+    };
+#pragma unroll
     for (uint32_t i = 0; i < kPer / 4; i++) {
-        uint4 x = v[i];
-        const uint32_t a = x.x, b = x.y, c = x.z, d = x.w;
-        x.x = run;
-        x.y = run + a;
-        x.z = run + a + b;
-        x.w = run + a + b + c;
-        run += a + b + c + d;
-        v[i] = x;
+#pragma unroll
+        for (uint32_t c = 0; c < kBinCounters; c++) take(v[c][i].x);
+#pragma unroll
+        for (uint32_t c = 0; c < kBinCounters; c++) take(v[c][i].y);
+#pragma unroll
+        for (uint32_t c = 0; c < kBinCounters; c++) take(v[c][i].z);
+#pragma unroll
+        for (uint32_t c = 0; c < kBinCounters; c++) take(v[c][i].w);
     }
+#pragma unroll
+    for (uint32_t c = 0; c < kBinCounters; c++)
+#pragma unroll
+        for (uint32_t i = 0; i < kPer / 4; i++)
+            reinterpret_cast<uint4*>(bins + c * kRayBins)[threadIdx.x * (kPer / 4) + i] = v[c][i];
 }
 
 // the bins' traversal order, from the mean walk of their rays since the last reorder (at most once
@@ -1513,7 +1527,7 @@ __global__ void __launch_bounds__(256) k_ray_bins_scatter(RayQueue q) {
     const uint32_t qi = grid_tid();
     if (qi >= q.counters[0]) return;
     const uint2 kr = q.key[qi];
-    q.perm[q.bins[kr.x] + kr.y] = qi;
+    q.perm[q.bins[(kr.x >> 16) * kRayBins + (kr.x & 0xFFFFu)] + kr.y] = qi;
 }
 
 // trace: persistent warps; a lane whose ray finished fetches the next one from the queue, so
@@ -1678,7 +1692,7 @@ __global__ void __launch_bounds__(128, 9) k_trace_photons(LaunchSet ls, RayQueue
         }
         if (finished) {
             q.hit[idx] = make_float4(__int_as_float(h.tri), h.bu, h.bv, h.bw);
-            if (q.perm) bin_cost_add(q, q.key[idx].x, (uint32_t)steps);
+            if (q.perm) bin_cost_add(q, q.key[idx].x & 0xFFFFu, (uint32_t)steps);
             if (COUNT) tc_segs++;
             idx = kNeed;
         }
@@ -2056,7 +2070,7 @@ void launch_gather_states(const JobDesc* jobs, const StateGather& list, JobState
     if (list.n) k_gather_states<<<list.n, 64, 0, s>>>(jobs, list, out);
 }
 void launch_frame_begin(const LaunchSet& ls, const RayQueue& q, cudaStream_t s) {
-    const uint32_t n = q.bins && ls.total < kRayBins ? kRayBins : ls.total;
+    const uint32_t n = q.bins && ls.total < kBinCounters * kRayBins ? kBinCounters * kRayBins : ls.total;
     if (ls.total) k_frame_begin<<<blocks_for(n, 256), 256, 0, s>>>(ls, q);
 }
 // block sizes: a multiple of 32 up to the kernel's launch bound (0 or anything else: the bound)
@@ -2102,7 +2116,7 @@ void launch_photon_gen_fp32(const LaunchSet& ls, const RayQueue& q, bool texture
     else k_photon_gen<false><<<blocks_for(n, 128), 128, 0, s>>>(ls, q);
 }
 void launch_queue_reset(const RayQueue& q, cudaStream_t s) {
-    if (q.counters) k_queue_reset<<<blocks_for(kRayBins, 256), 256, 0, s>>>(q);
+    if (q.counters) k_queue_reset<<<blocks_for(kBinCounters * kRayBins, 256), 256, 0, s>>>(q);
 }
 void launch_ray_bins_order(const RayQueue& q, cudaStream_t s) {
     if (q.key && q.bin_rank && q.bin_cost) k_ray_bins_order<<<1, 1024, 0, s>>>(q);

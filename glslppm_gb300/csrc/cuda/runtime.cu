@@ -985,8 +985,8 @@ int Runner::rebuild() {
         const size_t c = std::max<uint32_t>(cap, 1);
         size_t bytes = 3 * Arena::align(c * 16) + Arena::align(64) + Arena::align(c * 4) +
                        Arena::align(kEyeDeferred * 4) + Arena::align(c * 4) + Arena::align(c * 16);
-        if (binned) bytes += Arena::align(c * 8) + Arena::align(c * 4) + 2 * Arena::align(kRayBins * 4) +
-                             Arena::align(kRayBins * 8);
+        if (binned) bytes += Arena::align(c * 8) + Arena::align(c * 4) + Arena::align(kBinCounters * kRayBins * 4) +
+                             Arena::align(kRayBins * 4) + Arena::align(kRayBins * 8);
         if ((st = queue_mem.reserve(bytes))) return st;
         Arena& a = queue_mem;
         queue = RayQueue{};
@@ -1001,7 +1001,7 @@ int Runner::rebuild() {
         if (binned) {
             queue.key = a.take<uint2>(c);
             queue.perm = a.take<uint32_t>(c);
-            queue.bins = a.take<uint32_t>(kRayBins);
+            queue.bins = a.take<uint32_t>(kBinCounters * kRayBins);
             // bins traced in their own order until the first reorder
             queue.bin_rank = a.take<uint32_t>(kRayBins);
             queue.bin_cost = a.take<unsigned long long>(kRayBins);
