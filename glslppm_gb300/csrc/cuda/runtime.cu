@@ -1075,6 +1075,20 @@ void Runner::timed(int stage, bool start, cudaStream_t s) {
     }
 }
 
+// The order of the rays until the shapes are set.  Binning costs three more kernels and the ranks in the
+// generation (16 to 23 us and a few per cent of it); what it saves grows with the rays of one scene.
+// Measured (us a pass, binned / queue order, 512^2 images): Cornell box 122 / 108 at 2^17 slots, 192 / 187
+// at 2^19, 277 / 295 at 2^20; 102k-triangle mesh 423 / 394 at 2^19 and 1M triangles 1071 / 1132 at 2^21;
+// 16 jobs of 12k to 100k triangles 1114 / 1058.  The 4-wide walk, which takes the nearest child first, gains
+// nothing from bins: Cornell box 352 / 346 (2^20), 1M-triangle mesh 1242 / 937 (2^21), refilled every
+// 4 steps (8 steps: 964).
+constexpr uint32_t kBinnedSlots = 768 * 1024;
+constexpr uint32_t kMixedQueueRefill = 4;
+bool Runner::rays_in_queue_order() const {
+    if (shapes_set) return tune.unbinned_rays != 0;
+    return precision == SPPM_PRECISION_MIXED || active.size() > 1 || pho.total < kBinnedSlots;
+}
+
 void Runner::wait_resolve(cudaStream_t s) {
     // in a capture, an external event-wait node: each replay waits for the event's last record
     // before the replay's launch
@@ -1088,7 +1102,9 @@ int Runner::enqueue_frame(uint32_t phase) {
     RayQueue q = queue;
     q.refill_steps = tune.trace_refill_steps;
     q.tail_lanes = tune.trace_tail_lanes;
-    if (tune.unbinned_rays) {
+    const bool queue_order = rays_in_queue_order();
+    if (!q.refill_steps && queue_order && precision == SPPM_PRECISION_MIXED) q.refill_steps = kMixedQueueRefill;
+    if (queue_order) {
         q.key = nullptr;
         q.perm = nullptr;
         q.bins = nullptr;
@@ -1313,6 +1329,7 @@ int Runner::set_tuning(const sppm_tuning* t) {
     SPPM_CK(cudaSetDevice(device));
     SPPM_CK(cudaStreamSynchronize(stream));
     tune = *t;
+    shapes_set = true;
     trace_blocks = sms * (tune.trace_blocks_per_sm ? tune.trace_blocks_per_sm : trace_fit);
     drop_graphs();
     return SPPM_OK;

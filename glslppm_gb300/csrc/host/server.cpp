@@ -292,7 +292,9 @@ int sppm_server_create(const sppm_server_config* cfg, int device, sppm_server** 
     s->cfg = *cfg;
     int st = sppm_batch_create(&cfg->batch, device, &s->batch);
     if (st) return st;
-    if ((st = sppm_batch_set_tuning(s->batch, &cfg->tuning))) {
+    const sppm_tuning defaults{};  // zeros: the batch keeps its own
+    if (memcmp(&cfg->tuning, &defaults, sizeof(defaults)) != 0 &&
+        (st = sppm_batch_set_tuning(s->batch, &cfg->tuning))) {
         sppm_batch_destroy(s->batch);
         return st;
     }

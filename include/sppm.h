@@ -342,11 +342,15 @@ typedef struct sppm_tuning {
     uint32_t trace_blocks_per_sm; /* resident blocks of the persistent photon traversal per SM
                                      (0 = as many as fit)                                       */
     uint32_t trace_refill_steps;  /* traversal steps a warp takes before it refills its idle
-                                     lanes from the ray queue (0 = 32; 4-wide traversal 8)      */
+                                     lanes from the ray queue (0 = 32; 4-wide traversal 8, or 4
+                                     on the mixed path's rays in queue order)                   */
     uint32_t eye_block;           /* threads per block of the eye pass (0 = 128; 32..128)       */
     uint32_t store_block;         /* of the photon store + hash insertion (0 = 128; 32..128)    */
     uint32_t gather_block;        /* of the gather + progressive update (0 = 256; 32..256)      */
-    uint32_t unbinned_rays;       /* 1: photon rays traced in queue order instead of binned     */
+    uint32_t unbinned_rays;       /* 1: photon rays traced in queue order instead of binned.  Until
+                                     shapes are set the library chooses (and reports 0): bins for
+                                     the plain path's single job with 3/4 * 2^20 photon slots or
+                                     more, else queue order (same results)                      */
     uint32_t trace_tail_lanes;    /* exact traversal: once the ray queue is drained, a warp with
                                      at most this many walking lanes hands those walks to a tail
                                      kernel that finishes each with all 32 lanes of a warp (the
@@ -470,7 +474,8 @@ int sppm_debug_photon_rays(sppm_ctx* ctx, float* org, float* dir, uint32_t* phot
    fixed.  With offsets and records null only *num_records is set. */
 int sppm_debug_photon_grid(sppm_ctx* ctx, uint32_t* offsets, size_t offsets_capacity, uint32_t* records,
                            size_t records_capacity, uint32_t* num_records);
-/* The order the photon traversal takes the ray bins in (contexts with binned rays).  A ray's bin
+/* The order the photon traversal takes the ray bins in (contexts with binned rays; until a frame
+   has binned them, bin order and no costs).  A ray's bin
    is its direction class (cube face of the direction x the signs of its two minor components,
    24) x its origin cell (8^3 cells of the scene's bounding sphere, Morton-ordered): bin =
    class * 512 + cell.  rank[bin] = the bin's position in the traversal order; cost[position] =
