@@ -395,7 +395,12 @@ int sppm_debug_ray_bins(sppm_ctx* c, uint32_t* rank, uint64_t* cost, size_t capa
     if (!rank || !cost) return fail(SPPM_ERR_ARG, "null argument");
     if (capacity < kRayBins) return fail(SPPM_ERR_ARG, "capacity %zu < %u bins", capacity, kRayBins);
     SPPM_CK(cudaMemcpy(rank, q.bin_rank, (size_t)kRayBins * 4, cudaMemcpyDeviceToHost));
-    SPPM_CK(cudaMemcpy(cost, q.bin_cost, (size_t)kRayBins * 8, cudaMemcpyDeviceToHost));
+    std::vector<unsigned long long> parts((size_t)kBinCosts * kRayBins);
+    SPPM_CK(cudaMemcpy(parts.data(), q.bin_cost, parts.size() * 8, cudaMemcpyDeviceToHost));
+    for (uint32_t b = 0; b < kRayBins; b++) {
+        cost[b] = 0;
+        for (uint32_t k = 0; k < kBinCosts; k++) cost[b] += parts[(size_t)k * kRayBins + b];
+    }
     return SPPM_OK;
 }
 

@@ -172,6 +172,9 @@ constexpr uint32_t kRayBins = kRayDirClasses << (3 * kRayCellBits);
 // generation takes 291 / 210 / 208 us on a 1M-triangle mesh (2^21 slots, beside the eye pass every 10th
 // frame) and the one-block scan of the counters 10 / 12 / 16 us with the scatter of 2^16 rays.
 constexpr uint32_t kBinCounters = 2;
+// copies of the costs below, the traversal's blocks taking turns: the walks that end at one time are of
+// a few bins (the 4-wide walk on the mesh above, binned: 775 us a launch with one copy, 628 with two)
+constexpr uint32_t kBinCosts = 2;
 // eye pixels whose path the exact eye pass defers to its block-wide pass per frame (beyond it
 // the per-thread walk traces them)
 constexpr uint32_t kEyeDeferred = 4096;
@@ -195,7 +198,7 @@ struct RayQueue {
     // word and the index into bins); bin_cost[position] = (node steps << 32) + rays, summed by the
     // traversal since the last reorder, which puts the bins of the longest mean walks first
     uint32_t* bin_rank;             // [kRayBins]
-    unsigned long long* bin_cost;   // [kRayBins]
+    unsigned long long* bin_cost;   // [kBinCosts][kRayBins], the cost their sum
     uint32_t* perm;       // [capacity] queue index of the i-th ray in bin order
     uint32_t* eye_deferred;  // [kEyeDeferred] launch indices of the deferred eye pixels
     uint32_t refill_steps;   // traversal steps a warp takes between refills of its idle lanes
@@ -211,7 +214,8 @@ __device__ __forceinline__ void bin_cost_add(const RayQueue& q, uint32_t bin, ui
     const unsigned same = __match_any_sync(__activemask(), bin);
     const uint32_t sum = __reduce_add_sync(same, steps);
     if ((int)(threadIdx.x & 31) == __ffs(same) - 1) {
-        uint32_t* c = reinterpret_cast<uint32_t*>(q.bin_cost + bin);  // (steps << 32) + rays
+        // (steps << 32) + rays
+        uint32_t* c = reinterpret_cast<uint32_t*>(q.bin_cost + (blockIdx.x % kBinCosts) * kRayBins + bin);
         atomicAdd(c, (uint32_t)__popc(same));
         atomicAdd(c + 1, sum);
     }

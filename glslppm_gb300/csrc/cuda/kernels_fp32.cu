@@ -19,6 +19,7 @@
 //   k_gather             progressive.fs
 //   k_resolve            re.fs (on demand)
 // k_photon is the single-kernel form of gen + trace + store (SPPM_FLAG_FUSED_PHOTON).
+#include <cstddef>
 #include <cstdint>
 
 #include "bvh4_trace.cuh"
@@ -661,9 +662,12 @@ __device__ __forceinline__ void warp_bbox_atomics(JobState* st, f3 p, int job_k)
         uint32_t kmn = ok ? float_key(v[c]) : 0xFFFFFFFFu;
         kmx = __reduce_max_sync(mask, kmx);
         kmn = __reduce_min_sync(mask, kmn);
+        // An add to one address takes the GPU 0.7 ns, so six per warp were 137 us of the eye pass at
+        // 1024^2.  The bounds only grow: one read earlier (also a stale one, from L1) that already holds
+        // the warp's bounds makes the atomic unnecessary, as for nearly all warps.
         if ((threadIdx.x & 31) == (__ffs(mask) - 1)) {
-            atomicMax(&st->bbmax_key[c], kmx);
-            atomicMin(&st->bbmin_key[c], kmn);
+            if (kmx > __ldca(&st->bbmax_key[c])) atomicMax(&st->bbmax_key[c], kmx);
+            if (kmn < __ldca(&st->bbmin_key[c])) atomicMin(&st->bbmin_key[c], kmn);
         }
     }
 }
@@ -827,6 +831,12 @@ __device__ __forceinline__ void eye_write(const JobDesc& J, const JobState* st, 
 template <bool MIXED, bool TEX>
 __global__ void __launch_bounds__(128) k_eye(LaunchSet ls, uint32_t* deferred_n, uint32_t* deferred,
                                                 uint32_t deferred_cap) {
+    // the block's segment count for the job of its first item: one global add per block, made by the
+    // last of its threads to get there (no barrier: the others' registers are free when their paths
+    // have ended; lanes of one warp may get there apart)
+    __shared__ uint32_t s_segs, s_threads;
+    if (threadIdx.x == 0) s_segs = s_threads = 0u;
+    __syncthreads();
     const uint32_t g = grid_tid();
     if (g >= ls.total) return;
     const int k = find_job(ls, g);
@@ -853,13 +863,27 @@ __global__ void __launch_bounds__(128) k_eye(LaunchSet ls, uint32_t* deferred_n,
     if (done) eye_write(J, st, p, o);
     const f3 bpos = done ? o.pos : mk(__int_as_float(0x7FC00000), __int_as_float(0x7FC00000), __int_as_float(0x7FC00000));
     warp_bbox_atomics(st, bpos, k);  // a deferred pixel contributes nothing (NaN is ignored)
-    // segment count and errors: one atomic per warp and job
-    const unsigned mask = __match_any_sync(__activemask(), k);
+    // segment count and errors: one add per warp and job
+    const unsigned active = __activemask();
+    const unsigned mask = __match_any_sync(active, k);
     const uint32_t wsegs = __reduce_add_sync(mask, done ? o.segs : 0u);
     const uint32_t werr = __reduce_or_sync(mask, err);
+    const uint32_t first = blockIdx.x * blockDim.x;
+    const int block_k = find_job(ls, first);
     if ((threadIdx.x & 31) == (__ffs(mask) - 1)) {
-        atomicAdd(&st->eye_segments, (unsigned long long)wsegs);
+        if (k == block_k) atomicAdd(&s_segs, wsegs);
+        else atomicAdd(&st->eye_segments, (unsigned long long)wsegs);
         if (werr) atomicOr(&st->err, werr);
+    }
+    __syncwarp(active);
+    if ((threadIdx.x & 31) == (__ffs(active) - 1)) {
+        __threadfence_block();
+        const uint32_t n_active = __popc(active);
+        if (atomicAdd(&s_threads, n_active) + n_active == min(blockDim.x, ls.total - first)) {
+            __threadfence_block();
+            const uint32_t n = atomicAdd(&s_segs, 0u);
+            if (n) atomicAdd(&job_of(ls, block_k).state->eye_segments, (unsigned long long)n);
+        }
     }
 }
 
@@ -1295,7 +1319,8 @@ __global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
     __shared__ uint32_t order[128];
     __shared__ int2 rec_hit[128];
     __shared__ float4 rec_pos[128], rec_flux[128], rec_dir[128], rec_rng[128];
-    __shared__ uint32_t warp_emit[4], warp_valid[4];
+    __shared__ uint32_t warp_emit[4], warp_valid[4], warp_rays[4], block_base;
+    __shared__ int block_job;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     {
         const uint32_t g0 = ls.first + grid_tid();
@@ -1305,6 +1330,7 @@ __global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
         float4 pp, pf, pd, rn;
         if (valid) {
             const int k0 = find_job(ls, g0);
+            if (threadIdx.x == 0) block_job = k0;
             const JobDesc& J0 = job_of(ls, k0);
             const JobState* st0 = J0.state;
             const uint32_t s0 = g0 - first_item(ls, k0);
@@ -1342,47 +1368,70 @@ __global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
             rec_rng[dst] = rn;
         }
         __syncthreads();
-        if (threadIdx.x >= warp_valid[0] + warp_valid[1] + warp_valid[2] + warp_valid[3]) return;
     }
-    const uint32_t g = order[threadIdx.x];
-    const int k = find_job(ls, g);
+    // Every count of the pass is one address for all warps, and the GPU adds to one address once in 0.7 ns:
+    // with a ray count, an emission count and a segment count per warp, 2^20 slots took 46 to 69 us of
+    // the kernel's 75.  So a block adds once to the queue and once to its job's two counts.
+    constexpr unsigned kFull = 0xFFFFFFFFu;
+    const uint32_t t = threadIdx.x;
+    const bool on = t < warp_valid[0] + warp_valid[1] + warp_valid[2] + warp_valid[3];
+    const uint32_t g = on ? order[t] : 0u;
+    const int k = on ? find_job(ls, g) : block_job;
     const JobDesc& J = job_of(ls, k);
     JobState* st = J.state;
-    const uint32_t sidx = g - first_item(ls, k);
     uint32_t err = 0;
-    const uint32_t t = threadIdx.x;
-    float4 rndv = rec_rng[t];
-    const PhotonRay R = photon_generate<TEX>(J, rec_hit[t], rec_pos[t], rec_flux[t], rec_dir[t], rndv, err);
-    J.ph.rng[sidx] = rndv;
-    if (R.cont) {
-        J.ph.flux[sidx] = f4(R.flux, 0.0f);  // flux before the segment, read back by k_photon_store
-        J.ph.hit[sidx] = make_int2(-1, (int)R.depth);
-    } else {
-        photon_terminate(J, sidx);
-    }
-    const unsigned active = __activemask();
-    const unsigned live = __ballot_sync(active, R.cont);
-    uint32_t base = 0;
-    const int leader = __ffs(active) - 1;
-    if ((int)(threadIdx.x & 31) == leader && live) base = atomicAdd(&q.counters[0], __popc(live));
-    base = __shfl_sync(active, base, leader);
-    if (R.cont) {
-        const uint32_t qi = base + __popc(live & ((1u << (threadIdx.x & 31)) - 1));
-        q.org[qi] = make_float4(R.org.x, R.org.y, R.org.z, __uint_as_float(g));
-        q.dir[qi] = make_float4(R.dir.x, R.dir.y, R.dir.z, 0.0f);
-        if (q.key) {
-            // lanes with the same bin take consecutive ranks from one atomic
-            const uint32_t bin = q.bin_rank[ray_bin(J.scene, R.org, R.dir)];
-            const unsigned same = __match_any_sync(live, bin);
-            const int lead = __ffs(same) - 1;
-            uint32_t rb = 0;
-            const uint32_t counter = blockIdx.x % kBinCounters;
-            if ((int)(threadIdx.x & 31) == lead) rb = atomicAdd(&q.bins[counter * kRayBins + bin], __popc(same));
-            rb = __shfl_sync(same, rb, lead);
-            q.key[qi] = make_uint2(bin | counter << 16, rb + __popc(same & ((1u << (threadIdx.x & 31)) - 1)));
+    PhotonRay R;
+    R.cont = false;
+    R.emitted = 0;
+    uint32_t bin = 0, rank = 0;
+    if (on) {
+        const uint32_t sidx = g - first_item(ls, k);
+        float4 rndv = rec_rng[t];
+        R = photon_generate<TEX>(J, rec_hit[t], rec_pos[t], rec_flux[t], rec_dir[t], rndv, err);
+        J.ph.rng[sidx] = rndv;
+        if (R.cont) {
+            J.ph.flux[sidx] = f4(R.flux, 0.0f);  // flux before the segment, read back by k_photon_store
+            J.ph.hit[sidx] = make_int2(-1, (int)R.depth);
+        } else {
+            photon_terminate(J, sidx);
         }
     }
-    photon_counters(st, k, active, R.emitted, R.cont ? 1u : 0u, err);
+    const unsigned live = __ballot_sync(kFull, R.cont);
+    if (lane == 0) warp_rays[warp] = __popc(live);
+    const uint32_t emitted = __popc(__ballot_sync(kFull, R.emitted != 0));
+    if (lane == 0) warp_emit[warp] = emitted;
+    if (q.key && R.cont) {
+        // lanes with the same bin take consecutive ranks from one atomic
+        bin = q.bin_rank[ray_bin(J.scene, R.org, R.dir)];
+        const unsigned same = __match_any_sync(live, bin);
+        const int lead = __ffs(same) - 1;
+        const uint32_t counter = blockIdx.x % kBinCounters;
+        if ((int)lane == lead) rank = atomicAdd(&q.bins[counter * kRayBins + bin], __popc(same));
+        rank = __shfl_sync(same, rank, lead) + __popc(same & ((1u << lane) - 1u));
+        bin |= counter << 16;
+    }
+    const bool one_job = __syncthreads_and(!on || k == block_job) != 0;
+    if (t == 0) {
+        const uint32_t rays = warp_rays[0] + warp_rays[1] + warp_rays[2] + warp_rays[3];
+        block_base = rays ? atomicAdd(&q.counters[0], rays) : 0u;
+        if (one_job) {
+            // emitted_frame in the low word, segments_frame in the high one
+            static_assert(offsetof(JobState, emitted_frame) % 8 == 0 &&
+                          offsetof(JobState, segments_frame) == offsetof(JobState, emitted_frame) + 4, "one 64-bit add");
+            const unsigned long long n = (unsigned long long)rays << 32 | (warp_emit[0] + warp_emit[1] + warp_emit[2] + warp_emit[3]);
+            if (n) atomicAdd(reinterpret_cast<unsigned long long*>(&st->emitted_frame), n);
+        }
+    }
+    if (err) atomicOr(&st->err, err);
+    __syncthreads();
+    if (R.cont) {
+        uint32_t qi = block_base + __popc(live & ((1u << lane) - 1u));
+        for (uint32_t w = 0; w < warp; w++) qi += warp_rays[w];
+        q.org[qi] = make_float4(R.org.x, R.org.y, R.org.z, __uint_as_float(g));
+        q.dir[qi] = make_float4(R.dir.x, R.dir.y, R.dir.z, 0.0f);
+        if (q.key) q.key[qi] = make_uint2(bin, rank);
+    }
+    if (!one_job && on) photon_counters(st, k, __activemask(), R.emitted, R.cont ? 1u : 0u, 0u);
 }
 
 // exclusive scan of the bin counts in place, a bin's counters one after the other (one block of 1024
@@ -1468,7 +1517,10 @@ __global__ void __launch_bounds__(1024) k_ray_bins_order(RayQueue q) {
     uint32_t key[kRounds];
 #pragma unroll
     for (uint32_t r = 0; r < kRounds; r++) {
-        const unsigned long long c = q.bin_cost[q.bin_rank[r * 1024 + t]];
+        const uint32_t at = q.bin_rank[r * 1024 + t];
+        unsigned long long c = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < kBinCosts; k++) c += q.bin_cost[k * kRayBins + at];
         const uint32_t n = (uint32_t)c, mean = n ? (uint32_t)(c >> 32) / n : 0u;
         const uint32_t k = n ? 1u + min(254u, mean < 128u ? mean : 128u + (mean - 128u) / 8u) : 0u;
         key[r] = kKeys - 1u - k;  // descending mean
@@ -1495,7 +1547,7 @@ __global__ void __launch_bounds__(1024) k_ray_bins_order(RayQueue q) {
             run += v[i];
         }
     }
-    for (uint32_t i = t; i < kRayBins; i += 1024) q.bin_cost[i] = 0ull;  // every cost was read above
+    for (uint32_t i = t; i < kBinCosts * kRayBins; i += 1024) q.bin_cost[i] = 0ull;  // every cost was read above
     uint32_t rank[kRounds];
 #pragma unroll
     for (uint32_t r = 0; r < kRounds; r++) {

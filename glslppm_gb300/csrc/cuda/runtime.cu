@@ -986,7 +986,7 @@ int Runner::rebuild() {
         size_t bytes = 3 * Arena::align(c * 16) + Arena::align(64) + Arena::align(c * 4) +
                        Arena::align(kEyeDeferred * 4) + Arena::align(c * 4) + Arena::align(c * 16);
         if (binned) bytes += Arena::align(c * 8) + Arena::align(c * 4) + Arena::align(kBinCounters * kRayBins * 4) +
-                             Arena::align(kRayBins * 4) + Arena::align(kRayBins * 8);
+                             Arena::align(kRayBins * 4) + Arena::align(kBinCosts * kRayBins * 8);
         if ((st = queue_mem.reserve(bytes))) return st;
         Arena& a = queue_mem;
         queue = RayQueue{};
@@ -1004,11 +1004,11 @@ int Runner::rebuild() {
             queue.bins = a.take<uint32_t>(kBinCounters * kRayBins);
             // bins traced in their own order until the first reorder
             queue.bin_rank = a.take<uint32_t>(kRayBins);
-            queue.bin_cost = a.take<unsigned long long>(kRayBins);
+            queue.bin_cost = a.take<unsigned long long>(kBinCosts * kRayBins);
             std::vector<uint32_t> ident(kRayBins);
             for (uint32_t i = 0; i < kRayBins; i++) ident[i] = i;
             SPPM_CK(cudaMemcpy(queue.bin_rank, ident.data(), kRayBins * 4, cudaMemcpyHostToDevice));
-            SPPM_CK(cudaMemset(queue.bin_cost, 0, kRayBins * 8));
+            SPPM_CK(cudaMemset(queue.bin_cost, 0, kBinCosts * kRayBins * 8));
         }
         queue.capacity = (uint32_t)c;
         SPPM_CK(cudaMemset(queue.counters, 0, 64));
