@@ -502,15 +502,17 @@ struct Shade {
 // Result of raytrace() for a hit (eyeraytrace.fs:256-287)
 __device__ __forceinline__ Shade shade_hit(const DevScene& s, const Hit& h) {
     const float4* ts = s.tri_shade + (size_t)h.tri * 6;
-    const float4 r0 = __ldg(ts + 0), r1 = __ldg(ts + 1), r2 = __ldg(ts + 2);
-    const float4 r3 = __ldg(ts + 3), r4 = __ldg(ts + 4), r5 = __ldg(ts + 5);
+    float4 r0, r1, r2, r3, r4, r5;
+    ldg32(ts, r0, r1);
+    ldg32(ts + 2, r2, r3);
+    ldg32(ts + 4, r4, r5);
     const f3 V0 = mk(r1.x, r1.y, r1.z), V1 = mk(r1.w, r2.x, r2.y), V2 = mk(r2.z, r2.w, r3.x);
     const f3 N0 = mk(r3.y, r3.z, r3.w), N1 = mk(r4.x, r4.y, r4.z), N2 = mk(r4.w, r5.x, r5.y);
     Shade o;
     o.pos = add(add(scl(V2, h.bu), scl(V0, h.bv)), scl(V1, h.bw));
     o.nrm = normalize(add(add(scl(N2, h.bu), scl(N0, h.bv)), scl(N1, h.bw)));
     o.gnrm = mk(r0.x, r0.y, r0.z);
-    const DevMaterial& m = s.mats[h.mat];
+    const DevMaterial& m = s.mats[__float_as_int(r0.w)];
     o.col = mk(m.color[0], m.color[1], m.color[2]);
     o.brdf = m.brdf;
     o.eta = m.eta;
@@ -1831,7 +1833,6 @@ __global__ void __launch_bounds__(128) k_photon_store(LaunchSet ls, RayQueue q, 
     h.bu = hr.y;
     h.bv = hr.z;
     h.bw = hr.w;
-    h.mat = h.tri >= 0 ? __float_as_int(__ldg(&J.scene.tri_isect[(size_t)h.tri * 3 + 2]).y) : -1;
     const float4 f = J.ph.flux[sidx];
     const int depth = J.ph.hit[sidx].y;
     const uint32_t slot = photon_store(J, st, sidx, h, mk(d.x, d.y, d.z), mk(f.x, f.y, f.z), (float)depth, grid_shift);
