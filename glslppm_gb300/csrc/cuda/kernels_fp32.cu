@@ -826,13 +826,29 @@ __device__ __forceinline__ void eye_write(const JobDesc& J, const JobState* st, 
     J.px.emi_n[p] = qe;
 }
 
+// the pixel of item `item` of a job whose pixels a launch covers in 8x4 tiles (a warp's worth of items
+// each); false: the tile reaches over the image's edge there
+__device__ __forceinline__ bool tile_pixel(const JobDesc& J, uint32_t item, uint32_t& p) {
+    const uint32_t tw = (J.W + 7u) >> 3, tile = item >> 5, lane = item & 31u, ty = tile / tw;
+    const uint32_t px = (tile - ty * tw) * 8u + (lane & 7u), py = ty * 4u + (lane >> 3);
+    p = py * J.W + px;
+    return px < J.W && py < J.H;
+}
+
 // eye pass, one thread per pixel.  A ray with a zero direction component (slab_degenerate)
 // would walk most of the tree in one lane: the exact path defers such pixels to k_eye_coop
 // (their whole path is rerun there with block-wide walks); the mixed path's slab tests do not
 // degenerate.
+//
+// Bound by the divergence of a warp's paths and by the node loads' latency.  A warp takes an 8x4 tile:
+// its rays spread less than a row of 32 pixels does, so they share more nodes and end closer together.
+// Us a pass of ten with one eye frame, rows -> tiles: a 1024^2 frame of a 1M-triangle mesh 1057 -> 1049,
+// sixteen 512^2 frames 1043 -> 1029, the Cornell box at 1024^2 302 -> 301; and 8 resident blocks
+// (64 registers, 12 bytes spilled) 1049 -> 1044, 1029 -> 1025, 301 -> 301.  The textured path needs more
+// registers than that.
 template <bool MIXED, bool TEX>
-__global__ void __launch_bounds__(128) k_eye(LaunchSet ls, uint32_t* deferred_n, uint32_t* deferred,
-                                                uint32_t deferred_cap) {
+__global__ void __launch_bounds__(128, TEX ? 5 : 8)
+    k_eye(LaunchSet ls, uint32_t* deferred_n, uint32_t* deferred, uint32_t deferred_cap) {
     // the block's segment count for the job of its first item: one global add per block, made by the
     // last of its threads to get there (no barrier: the others' registers are free when their paths
     // have ended; lanes of one warp may get there apart)
@@ -844,10 +860,10 @@ __global__ void __launch_bounds__(128) k_eye(LaunchSet ls, uint32_t* deferred_n,
     const int k = find_job(ls, g);
     const JobDesc& J = job_of(ls, k);
     JobState* st = J.state;
-    const uint32_t p = g - first_item(ls, k);
-    uint32_t err = 0;
+    uint32_t p, err = 0;
     EyeOut o;
-    const bool done = eye_path<TEX>(J, st, p, [&](f3 org, f3 dir, bool cull, Hit& h) {
+    const bool live = tile_pixel(J, g - first_item(ls, k), p);
+    const bool done = live && eye_path<TEX>(J, st, p, [&](f3 org, f3 dir, bool cull, Hit& h) {
         if (MIXED) {
             h = trace_eye4(J.scene, org, dir, cull, err);
             return true;
@@ -901,8 +917,8 @@ __global__ void __launch_bounds__(kBlockWalk) k_eye_coop(LaunchSet ls, const uin
         const int k = find_job(ls, g);
         const JobDesc& J = job_of(ls, k);
         JobState* st = J.state;
-        const uint32_t p = g - first_item(ls, k);
-        uint32_t err = 0;
+        uint32_t p, err = 0;
+        tile_pixel(J, g - first_item(ls, k), p);
         EyeOut o;
         eye_path<TEX>(J, st, p, [&](f3 org, f3 dir, bool cull, Hit& h) {
             TraversalCount ct;
@@ -1853,11 +1869,9 @@ __global__ void __launch_bounds__(256, 4) k_gather(LaunchSet ls) {
     const int k = find_job(ls, g);
     const JobDesc& J = job_of(ls, k);
     JobState* st = J.state;
-    const uint32_t item = g - first_item(ls, k), lane = threadIdx.x & 31u;
-    const uint32_t tw = (J.W + 7u) >> 3, tile = item >> 5, ty = tile / tw;
-    const uint32_t px = (tile - ty * tw) * 8u + (lane & 7u), py = ty * 4u + (lane >> 3);
-    if (px >= J.W || py >= J.H) return;
-    const uint32_t p = py * J.W + px;
+    const uint32_t item = g - first_item(ls, k);
+    uint32_t p;
+    if (!tile_pixel(J, item, p)) return;
     const uint32_t frame = st->frame;
     if (p == 0) {
         // NumPhotons += int(sum) (glslppm.cpp:397) once the photon pass of this frame is done

@@ -907,6 +907,9 @@ void Runner::drop_graphs() {
 
 bool Runner::phase_has_eye(uint32_t phase) const { return phase < eye_pix.size() && eye_pix[phase].njobs > 0; }
 
+// the items of a job's pixels in 8x4 tiles, 32 each
+static uint64_t tile_items(const Job& j) { return 32ull * ((j.W + 7) / 8) * ((j.H + 3) / 4); }
+
 int Runner::rebuild() {
     SPPM_CK(cudaSetDevice(device));
     SPPM_CK(cudaStreamSynchronize(stream));
@@ -927,7 +930,7 @@ int Runner::rebuild() {
             acc += w == 0 ? j->npix
                  : w == 1 ? j->P
                  : w == 2 ? j->hash_num
-                          : 32ull * ((j->W + 7) / 8) * ((j->H + 3) / 4);
+                          : tile_items(*j);
         }
         t.push_back((uint32_t)acc);
         tot[w] = acc;
@@ -943,7 +946,7 @@ int Runner::rebuild() {
             if (j->eye_phase(L) != p) continue;
             ids.push_back(j->slot);
             pref.push_back((uint32_t)acc);
-            acc += j->npix;
+            acc += tile_items(*j);
         }
         pref.push_back((uint32_t)acc);
         eye_cnt[p] = ids.size();
@@ -974,7 +977,7 @@ int Runner::rebuild() {
         const uint32_t m = (uint32_t)eye_cnt[p];
         uint64_t px = 0;
         for (Job* j : active)
-            if (j->eye_phase(L) == p) px += j->npix;
+            if (j->eye_phase(L) == p) px += tile_items(*j);
         eye_pix[p] = mk(eye_off[p], eye_off[p] + m, m, px);
         eye_ids[p] = d_t + eye_off[p];
     }
