@@ -24,35 +24,44 @@ struct Hit4 {
 
 __device__ __forceinline__ float node_scale(uint8_t e) { return __uint_as_float((uint32_t)e << 23); }
 
-// direction component used for the slab reciprocals: a zero (or denormal-small) component is
-// replaced by +-1e-30 so that the slab of that axis is +-huge instead of NaN (a NaN slab would be
-// ignored by fminf/fmaxf and the ray would enter every box the other axes allow)
-__device__ __forceinline__ float slab_dir(float d) { return fabsf(d) < 1e-30f ? copysignf(1e-30f, d) : d; }
-
-// byte k of w as an exact float: the byte placed in the low mantissa of 2^23, minus 2^23
-__device__ __forceinline__ float byte_f(uint32_t w, uint32_t sel) {
-    return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)) - 8388608.0f;
-}
+// direction component used for the slab reciprocals: a zero (or tiny) component is replaced by
+// +-1e-26 so that the slab of that axis is +-huge instead of NaN (a NaN slab would be ignored by
+// fminf/fmaxf and the ray would enter every box the other axes allow)
+__device__ __forceinline__ float slab_dir(float d) { return fabsf(d) < 1e-26f ? copysignf(1e-26f, d) : d; }
 
 // ---- conservative slab tests over the quantised boxes ------------------------------------------
-// A child plane is P = origin + q * 2^e (q a byte); its distance along the ray is computed as
-//     fma(q, A, B -+ E),  A = 2^e * r (exact scaling of r = fl(1/d)),  B = fma(origin, r, n),
-//     n = fl(-o * r).
+// A child plane is P = origin + q * 2^e (q a byte).  One byte permutation places the byte in the
+// mantissa of 1.0: f = 1 + q * 2^-15, and the plane's distance along the ray is
+//     fma(f, A, B - A -+ E),  A = 2^(e+15) * r (exact scaling of r = fl(1/d)),
+//     B = fma(origin, r, n),  n = fl(-o * r),
+// the two planes of a child and axis in one two-lane operation (near with -E, far with +E): half the
+// instructions of q made a float of its own (permutation and subtraction) and two scalar fmas.
 // Against the exact distance (P' - o) / d to the enclosing plane P' = fl(origin + q 2^e) that the
-// builder checked, the roundings of r, n, B, B -+ E, the final fma and P' add at most
-// 5 u S (1 + O(u)), u = 2^-24, with S = (|origin| + |o| + 255 * 2^e) / |d|
-// (each rounding's error is u times a term bounded by S).  E = 16 u S', S' the same sum computed
-// from |r|, |n| and |A| (relative error a few u), exceeds that bound, so the near distance is never
-// above the exact entry and the far distance never below the exact exit: a box the exact
-// arithmetic enters is never culled (Ize, "Robust BVH Ray Traversal", JCGT 2013, applies the same
-// argument to the plain slab test).  The near plane of each axis is chosen by the sign of the
-// direction once per ray, so a child needs no per-axis min/max.
+// builder checked, the roundings of r, n, B, B - A, -+ E, the fma and P' add at most
+// 8 u S + 2^-8 * 2^e |r| (1 + O(u)), u = 2^-24, with S = (|origin| + |o| + 255 * 2^e) / |d| (each
+// rounding's error is u times a term bounded by S, and those of B - A and -+ E u times |A| more).
+// E = 16 u S' + 2^-7 * 2^e |r|, S' the same sum computed from |r|, |n| and |A| (relative error a few
+// u), exceeds that bound, so the near distance is never above the exact entry and the far distance
+// never below the exact exit: a box the exact arithmetic enters is never culled (Ize, "Robust BVH Ray
+// Traversal", JCGT 2013, applies the same argument to the plain slab test).  Where A overflows, the
+// distances become NaN, which the minimum and maximum drop: the box is entered.  The near plane of
+// each axis is chosen by the sign of the direction once per node, so a child needs no per-axis
+// min/max.
 constexpr float kSlabErr = 9.5367431640625e-07f;  // 16 * 2^-24
+// E's part in |A|: 255 * 2^-15 of S', and 2^-7 of a step (2^-22 of A)
+constexpr float kSlabErrA = 255.0f * kSlabErr / 32768.0f + 2.384185791015625e-07f;
 // a box entered later than the closest hit so far by less than this relative margin is still
 // visited: the exact triangle test's own rounding may put the winner's t just below its box entry
 constexpr float kCullMargin = 1.000244140625f;    // 1 + 2^-12
 
-// (|r| and |n| are free operand modifiers; r < 0 selects the upper bound as the near plane)
+// a * b + c in two single-precision lanes
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// (r < 0 selects the upper bound as the near plane)
 struct Ray4 {
     float ox, oy, oz, dx, dy, dz;
     float rx, ry, rz, nx, ny, nz;     // r = 1/slab_dir(d), n = -o * r
@@ -64,51 +73,44 @@ __device__ __forceinline__ void ray4_setup(Ray4& R, float ox, float oy, float oz
     R.nx = -ox * R.rx, R.ny = -oy * R.ry, R.nz = -oz * R.rz;
 }
 
-// the node's per-axis slab operands for one ray
+// one axis of a node for one ray
 struct Slab4 {
-    float Ax, Ay, Az;        // 2^e * r
-    float Nx, Ny, Nz;        // B - E (near planes)
-    float Fx, Fy, Fz;        // B + E (far planes)
-    uint32_t nwx, nwy, nwz;  // words holding the near-plane bytes of the four children
-    uint32_t fwx, fwy, fwz;  // ... and the far-plane bytes
+    unsigned long long A, B;  // A twice; B - A - E (near planes) and B - A + E (far planes)
+    uint32_t near, far;       // words holding the near-plane and far-plane bytes of the four children
 };
 
-__device__ __forceinline__ float slab_err(float origin, float r, float n, float A) {
-    return kSlabErr * fmaf(255.0f, fabsf(A), fmaf(fabsf(origin), fabsf(r), fabsf(n)));
+// e: the axis' exponent byte; lo, hi: the words of its lower and upper bytes
+__device__ __forceinline__ Slab4 slab4(uint32_t e, float origin, float lo, float hi, float r, float n) {
+    Slab4 s;
+    const float A = (node_scale(e) * r) * 32768.0f;
+    const float C = fmaf(origin, r, n) - A;
+    const float E = fmaf(kSlabErrA, fabsf(A), kSlabErr * fmaf(fabsf(origin), fabsf(r), fabsf(n)));
+    s.A = pack2(A, A);
+    s.B = pack2(C - E, C + E);
+    const bool neg = r < 0.0f;
+    s.near = __float_as_uint(neg ? hi : lo);
+    s.far = __float_as_uint(neg ? lo : hi);
+    return s;
 }
 
-__device__ __forceinline__ void slab4_setup(Slab4& S, const Ray4& R, const float4& w0, const float4& w2,
-                                            const float4& w3) {
-    const uint32_t eb = __float_as_uint(w0.w);
-    S.Ax = node_scale(eb & 0xFF) * R.rx;
-    S.Ay = node_scale((eb >> 8) & 0xFF) * R.ry;
-    S.Az = node_scale((eb >> 16) & 0xFF) * R.rz;
-    const float Bx = fmaf(w0.x, R.rx, R.nx), By = fmaf(w0.y, R.ry, R.ny), Bz = fmaf(w0.z, R.rz, R.nz);
-    const float Ex = slab_err(w0.x, R.rx, R.nx, S.Ax);
-    const float Ey = slab_err(w0.y, R.ry, R.ny, S.Ay);
-    const float Ez = slab_err(w0.z, R.rz, R.nz, S.Az);
-    S.Nx = Bx - Ex, S.Ny = By - Ey, S.Nz = Bz - Ez;
-    S.Fx = Bx + Ex, S.Fy = By + Ey, S.Fz = Bz + Ez;
-    // lower bytes: x w2.x, y w2.y, z w2.z; upper bytes: x w2.w, y w3.x, z w3.y
-    const uint32_t lx = __float_as_uint(w2.x), ly = __float_as_uint(w2.y), lz = __float_as_uint(w2.z);
-    const uint32_t hx = __float_as_uint(w2.w), hy = __float_as_uint(w3.x), hz = __float_as_uint(w3.y);
-    const bool negx = R.rx < 0.0f, negy = R.ry < 0.0f, negz = R.rz < 0.0f;
-    S.nwx = negx ? hx : lx, S.fwx = negx ? lx : hx;
-    S.nwy = negy ? hy : ly, S.fwy = negy ? ly : hy;
-    S.nwz = negz ? hz : lz, S.fwz = negz ? lz : hz;
+// near and far distance of child K along one axis
+template <int K>
+__device__ __forceinline__ void slab4_child(const Slab4& s, float& near, float& far) {
+    constexpr uint32_t sel = 0x7604u | ((uint32_t)K << 4);  // byte K under the exponent of 1.0
+    const float fn = __uint_as_float(__byte_perm(s.near, 0x3F800000u, sel));
+    const float ff = __uint_as_float(__byte_perm(s.far, 0x3F800000u, sel));
+    unpack2(fma2(pack2(fn, ff), s.A, s.B), near, far);
 }
 
 // conservative entry distance of child K (clamped at 0) and whether the ray may hit its box before
 // tcull (the closest hit so far times kCullMargin)
 template <int K>
-__device__ __forceinline__ void child_box(const Slab4& S, float tcull, float& tn, bool& hit) {
-    constexpr uint32_t sel = 0x7650u | (uint32_t)K;  // byte K of the word into byte 0, 0x4B into byte 3
-    const float nx = fmaf(byte_f(S.nwx, sel), S.Ax, S.Nx);
-    const float ny = fmaf(byte_f(S.nwy, sel), S.Ay, S.Ny);
-    const float nz = fmaf(byte_f(S.nwz, sel), S.Az, S.Nz);
-    const float fx = fmaf(byte_f(S.fwx, sel), S.Ax, S.Fx);
-    const float fy = fmaf(byte_f(S.fwy, sel), S.Ay, S.Fy);
-    const float fz = fmaf(byte_f(S.fwz, sel), S.Az, S.Fz);
+__device__ __forceinline__ void child_box(const Slab4& X, const Slab4& Y, const Slab4& Z, float tcull, float& tn,
+                                          bool& hit) {
+    float nx, ny, nz, fx, fy, fz;
+    slab4_child<K>(X, nx, fx);
+    slab4_child<K>(Y, ny, fy);
+    slab4_child<K>(Z, nz, fz);
     const float t0 = fmaxf(fmax3(nx, ny, nz), 0.0f);
     const float t1 = fmin3(fx, fy, fz);
     tn = t0;
@@ -159,13 +161,15 @@ __device__ __forceinline__ Hit4 trace4(const Node4Dev* __restrict__ nodes, const
         // conservative slab test of the (up to) four children
         float tnear[4];
         bool hit[4];
-        Slab4 S;
-        slab4_setup(S, R, w0, w2, w3);
+        const uint32_t eb = __float_as_uint(w0.w);
+        const Slab4 X = slab4(eb & 0xFF, w0.x, w2.x, w2.w, R.rx, R.nx);
+        const Slab4 Y = slab4((eb >> 8) & 0xFF, w0.y, w2.y, w3.x, R.ry, R.ny);
+        const Slab4 Z = slab4((eb >> 16) & 0xFF, w0.z, w2.z, w3.y, R.rz, R.nz);
         const float tcull = h.t * kCullMargin;
-        child_box<0>(S, tcull, tnear[0], hit[0]);
-        child_box<1>(S, tcull, tnear[1], hit[1]);
-        child_box<2>(S, tcull, tnear[2], hit[2]);
-        child_box<3>(S, tcull, tnear[3], hit[3]);
+        child_box<0>(X, Y, Z, tcull, tnear[0], hit[0]);
+        child_box<1>(X, Y, Z, tcull, tnear[1], hit[1]);
+        child_box<2>(X, Y, Z, tcull, tnear[2], hit[2]);
+        child_box<3>(X, Y, Z, tcull, tnear[3], hit[3]);
         // leaf children: their triangles in child order (a closer hit shrinks the search), one copy
         // of the test in a loop over the leaves
         uint32_t leaves = 0;

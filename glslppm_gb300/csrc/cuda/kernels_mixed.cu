@@ -44,15 +44,24 @@ __device__ __noinline__ bool met_first(const LaunchSet& ls, int job_k, const Ray
 // photon segments through the 4-wide BVH: persistent warps with dynamic ray fetch (a lane whose
 // ray finished takes the next queued ray), one node per lane per step, closest child first, the
 // other hit children on a per-thread stack in shared memory
+//
+// Bound by the instructions it issues (the walk's loads hit L1 and L2) and, in the larger trees, by
+// how many of a warp's lanes still walk.  So: two-lane slab tests (child_box), one 64-bit shared-memory
+// access per stack entry with one check of the space for all of a node's pushes, no compare that a
+// later one repeats, the triangle test left at the first coordinate that fails, and no jump out of
+// the inner loops (after one the compiler does not bring the warp's lanes together again before the
+// next node).  Us a pass, together: the Cornell box at 1024^2 324.7 -> 312.6, a 1M-triangle mesh at
+// 1024^2 891 -> 843; of which the slab test 6 and 16, the loops' form 3 and 11, the pushes and
+// compares 5 and 12, the triangle test 0 and 6.  64 registers, 8 blocks per SM by the stacks' shared
+// memory: 7 blocks 316 and 873, 10 with spills 346 and 973; a stack of 12 entries there 319 and 869
+// (of 24: 314 and 851).
 __global__ void __launch_bounds__(kTraceBlock) k_trace_photons4(LaunchSet ls, RayQueue q) {
-    __shared__ int32_t s_node[kSmemStack][kTraceBlock];
-    __shared__ float s_t[kSmemStack][kTraceBlock];
+    __shared__ int2 s_nt[kSmemStack][kTraceBlock];
     int32_t l_node[kLocalStack];
     float l_t[kLocalStack];
     auto push = [&](int sp_, int32_t n, float t) {
         if (sp_ < kSmemStack) {
-            s_node[sp_][threadIdx.x] = n;
-            s_t[sp_][threadIdx.x] = t;
+            s_nt[sp_][threadIdx.x] = make_int2(n, __float_as_int(t));
         } else {
             l_node[sp_ - kSmemStack] = n;
             l_t[sp_ - kSmemStack] = t;
@@ -121,24 +130,25 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_photons4(LaunchSet ls, Ra
             float4 w0, w1, w2, w3;
             ldg32(np, w0, w1);
             ldg32(np + 2, w2, w3);
-            const int cnt = (int)(__float_as_uint(w0.w) >> 24);
             float t[4];
             bool hit[4];
-            Slab4 S;
-            slab4_setup(S, R, w0, w2, w3);
+            const uint32_t eb = __float_as_uint(w0.w);
+            const Slab4 X = slab4(eb & 0xFF, w0.x, w2.x, w2.w, R.rx, R.nx);
+            const Slab4 Y = slab4((eb >> 8) & 0xFF, w0.y, w2.y, w3.x, R.ry, R.ny);
+            const Slab4 Z = slab4((eb >> 16) & 0xFF, w0.z, w2.z, w3.y, R.rz, R.nz);
             const float tcull = ht * kCullMargin;
-            child_box<0>(S, tcull, t[0], hit[0]);
-            child_box<1>(S, tcull, t[1], hit[1]);
-            child_box<2>(S, tcull, t[2], hit[2]);
-            child_box<3>(S, tcull, t[3], hit[3]);
+            child_box<0>(X, Y, Z, tcull, t[0], hit[0]);
+            child_box<1>(X, Y, Z, tcull, t[1], hit[1]);
+            child_box<2>(X, Y, Z, tcull, t[2], hit[2]);
+            child_box<3>(X, Y, Z, tcull, t[3], hit[3]);
             int32_t c[4] = {__float_as_int(w1.x), __float_as_int(w1.y), __float_as_int(w1.z), __float_as_int(w1.w)};
-            // leaf children hit: their triangles, in child order (photons pass through emitters);
-            // one copy of the test in a loop over the leaves, so a warp runs it as many times as
-            // its lane with the most leaves needs
+            // leaf children hit: their triangles, in child order (photons pass through emitters, and
+            // an empty child's link, all bits of ~link but the sign, reads as one); one copy of the
+            // test in a loop over the leaves, so a warp runs it as many times as its lane with the
+            // most leaves needs
             uint32_t leaves = 0;
 #pragma unroll
             for (int k = 0; k < 4; k++) {
-                hit[k] = hit[k] && k < cnt;
                 if (!hit[k] || c[k] >= 0) continue;
                 hit[k] = false;
                 if (!(~c[k] & kEmitterBit)) leaves |= 1u << k;
@@ -151,51 +161,69 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_photons4(LaunchSet ls, Ra
                 const float4 a = __ldg(&tri_isect[(size_t)code * 3 + 0]);
                 const float4 b = __ldg(&tri_isect[(size_t)code * 3 + 1]);
                 const float4 cc = __ldg(&tri_isect[(size_t)code * 3 + 2]);
-                float tt, u, v, w;
-                if (tri_hit_exact(a, b, cc, mk(R.ox, R.oy, R.oz), mk(R.dx, R.dy, R.dz), false, tt, u, v, w) &&
-                    (tt < ht || (tt == ht && htri >= 0 && met_first(ls, job_k, R, code, htri)))) {
-                    ht = tt;
-                    htri = code;
-                    hbu = v;
-                    hbv = w;
-                    hbw = u;
+                // tri_hit_exact's arithmetic; u > 1 leaves w < 0 whatever v is
+                const f3 dir = mk(R.dx, R.dy, R.dz);
+                const f3 e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, cc.x);
+                const f3 pv = cross(dir, e1);
+                const float det = dot(e0, pv);
+                const f3 tv = sub(mk(R.ox, R.oy, R.oz), mk(a.x, a.y, a.z));
+                const f3 qv = cross(tv, e0);
+                const float u = xdiv(dot(tv, pv), det);
+                if (u >= 0.0f && u <= 1.0f) {
+                    const float v = xdiv(dot(dir, qv), det);
+                    const float w = xsub(xsub(1.0f, u), v);
+                    if (v >= 0.0f && w >= 0.0f) {
+                        const float tt = xdiv(dot(e1, qv), det);
+                        if (tt >= 0.0f && (tt < ht || (tt == ht && htri >= 0 && met_first(ls, job_k, R, code, htri)))) {
+                            ht = tt;
+                            htri = code;
+                            hbu = v;
+                            hbv = w;
+                            hbw = u;
+                        }
+                    }
                 }
             }
-            // internal children hit before the current closest hit, sorted near to far
+            // internal children hit before the current closest hit, sorted near to far (a triangle
+            // above may have brought it closer than tcull)
             const float tcull2 = ht * kCullMargin;
 #pragma unroll
             for (int k = 0; k < 4; k++)
-                if (!(hit[k] && t[k] <= tcull2)) t[k] = __int_as_float(0x7f800000);
+                if (!hit[k]) t[k] = __int_as_float(0x7f800000);
             cswap(t[0], c[0], t[1], c[1]);
             cswap(t[2], c[2], t[3], c[3]);
             cswap(t[0], c[0], t[2], c[2]);
             cswap(t[1], c[1], t[3], c[3]);
             cswap(t[1], c[1], t[2], c[2]);
-            const float inf = __int_as_float(0x7f800000);
-            if (t[0] < inf) {
-                const int pushes = (t[1] < inf) + (t[2] < inf) + (t[3] < inf);
+            bool found = t[0] <= tcull2;
+            if (found) {
+                const int pushes = (t[1] <= tcull2) + (t[2] <= tcull2) + (t[3] <= tcull2);
                 if (sp + pushes > kStack) {
                     err |= kErrWatchdogTraverse;
-                    finished = true;
-                    break;
+                    found = false;
+                    sp = 0;
+                } else {
+                    if (sp + pushes <= kSmemStack) {
+                        if (t[3] <= tcull2) s_nt[sp++][tid] = make_int2(c[3], __float_as_int(t[3]));
+                        if (t[2] <= tcull2) s_nt[sp++][tid] = make_int2(c[2], __float_as_int(t[2]));
+                        if (t[1] <= tcull2) s_nt[sp++][tid] = make_int2(c[1], __float_as_int(t[1]));
+                    } else {
+                        if (t[3] <= tcull2) push(sp++, c[3], t[3]);
+                        if (t[2] <= tcull2) push(sp++, c[2], t[2]);
+                        if (t[1] <= tcull2) push(sp++, c[1], t[1]);
+                    }
+                    cur = c[0];
                 }
-                if (t[3] < inf) push(sp++, c[3], t[3]);
-                if (t[2] < inf) push(sp++, c[2], t[2]);
-                if (t[1] < inf) push(sp++, c[1], t[1]);
-                cur = c[0];
-                continue;
             }
-            bool found = false;
-            while (sp > 0) {
+            while (!found && sp > 0) {
                 sp--;
-                const float st_t = sp < kSmemStack ? s_t[sp][tid] : l_t[sp - kSmemStack];
-                if (st_t <= ht * kCullMargin) {
-                    cur = sp < kSmemStack ? s_node[sp][tid] : l_node[sp - kSmemStack];
-                    found = true;
-                    break;
-                }
+                int2 e;
+                if (sp < kSmemStack) e = s_nt[sp][tid];
+                else e = make_int2(l_node[sp - kSmemStack], __float_as_int(l_t[sp - kSmemStack]));
+                cur = e.x;
+                found = __int_as_float(e.y) <= ht * kCullMargin;
             }
-            if (!found) finished = true;
+            finished = !found;
         }
         if (finished) {
             q.hit[idx] = make_float4(__int_as_float(htri), hbu, hbv, hbw);
