@@ -415,6 +415,29 @@ __device__ __forceinline__ int cube_face(f3 d) {
     return d.z < 0.0f ? 5 : 4;
 }
 
+
+// Sine and cosine of one angle, |x| < 2^20: the operations of sppm_fsin and sppm_fcos, so the same
+// values, with one reduction for both and the quadrant taken by selection (the two calls reduce twice
+// and send a warp's four quadrants down four branches each).
+__device__ __forceinline__ void fsincos(float x, float& sn, float& cs) {
+    const float k = floorf(xadd(xmul(x, SPPM_FP_TWO_OVER_PI), 0.5f));
+    float r = xsub(x, xmul(k, SPPM_FP_PIO2_1));
+    r = xsub(r, xmul(k, SPPM_FP_PIO2_2));
+    r = xsub(r, xmul(k, SPPM_FP_PIO2_3));
+    const float r2 = xmul(r, r);
+    float ps = xsub(SPPM_FP_INV_7F, xmul(r2, SPPM_FP_INV_9F));
+    ps = xsub(SPPM_FP_INV_5F, xmul(r2, ps));
+    ps = xsub(SPPM_FP_INV_3F, xmul(r2, ps));
+    const float s = xsub(r, xmul(xmul(r, r2), ps));
+    float pc = xsub(SPPM_FP_INV_8F, xmul(r2, SPPM_FP_INV_10F));
+    pc = xsub(SPPM_FP_INV_6F, xmul(r2, pc));
+    pc = xsub(SPPM_FP_INV_4F, xmul(r2, pc));
+    const float c = xadd(xsub(1.0f, xmul(r2, SPPM_FP_INV_2F)), xmul(xmul(r2, r2), pc));
+    const int q = (int)k;
+    const float a = (q & 1) ? c : s, b = (q & 1) ? s : c;
+    sn = (q & 2) ? -a : a;
+    cs = ((q + 1) & 2) ? -b : b;
+}
 // ---- GPURnd (eyeraytrace.fs:326-347) and the cell hash (hash.fs:21-48) ---------------------
 // lane constants q, r, a, m and the single-precision 1/m, 1/q, m/2 the shaders derive from them
 #define SPPM_RND_LANE(i, q, r, a, m, qinv, minv)                                                \
@@ -449,11 +472,28 @@ __device__ __forceinline__ void schrage4(float s[4], float v[4]) {
     schrage_lane<3>(s, v);
 }
 
+// floor of |x| < 2^22: 1.5 * 2^23 has a spacing of 1 up to 2^24, so the sum rounded down is the floor
+// (two additions at the full rate; the conversion unit's floor has an eighth of it)
+__device__ __forceinline__ float floor_small(float x) { return xsub(__fadd_rd(x, 12582912.0f), 12582912.0f); }
+// One lane of the generator's step, SPPM_RND_LANE's values for a state of 0 <= s <= 2^22, which seeds and
+// outputs are: beta, an integer up to 2^22 / q, times q or r is exact, so the fused operations round as
+// the separate ones do; m / 2 is exact, so the addend is 0, m / 2 or m.  (hash_cell's lanes take any
+// cell and keep the general form.)  Us a pass, with fsincos: the Cornell box at 1024^2 301.6 -> 299.0,
+// sixteen jobs 1031 -> 1019, glass and glossy spheres with 517x389 photons 170.2 -> 163.7.
+__device__ __forceinline__ float rnd_lane(float& s, float q, float r, float a, float m, float qinv, float minv) {
+    const float beta = floor_small(xmul(s, qinv));
+    const float p = __fmaf_rn(-beta, r, xmul(a, __fmaf_rn(-beta, q, s)));
+    s = xadd(p, p > 0.0f ? 0.0f : (p < 0.0f ? m : 0.5f * m));
+    return xmul(s, minv);
+}
+
 __device__ __forceinline__ float gpu_rnd(float4& n) {
-    float s[4] = {n.x, n.y, n.z, n.w}, v[4];
-    schrage4(s, v);
-    n = make_float4(s[0], s[1], s[2], s[3]);
-    return fractf(xsub(xadd(xsub(v[0], v[1]), v[2]), v[3]));
+    const float v0 = rnd_lane(n.x, 1225.0f, 1112.0f, 3423.0f, 4194287.0f, 8.163265302e-04f, 2.384195454e-07f);
+    const float v1 = rnd_lane(n.y, 1585.0f, 367.0f, 2646.0f, 4194277.0f, 6.309148157e-04f, 2.384201139e-07f);
+    const float v2 = rnd_lane(n.z, 2457.0f, 92.0f, 1707.0f, 4194191.0f, 4.070004215e-04f, 2.384250024e-07f);
+    const float v3 = rnd_lane(n.w, 2098.0f, 265.0f, 1999.0f, 4194167.0f, 4.766444326e-04f, 2.384263666e-07f);
+    const float u = xsub(xadd(xsub(v0, v1), v2), v3);
+    return xsub(u, floor_small(u));
 }
 
 __device__ __forceinline__ uint32_t hash_cell(f3 cell, float grid_scale, float hash_scale1, float hash_num) {

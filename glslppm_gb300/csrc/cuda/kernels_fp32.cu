@@ -578,7 +578,9 @@ __device__ __forceinline__ f3 glossy_reflect(f3 d, f3 n, float g, float4& rndv) 
     const float temp1 = xmul(6.283184f, rnd1);
     const float temp2_ = sppm_fpow(rnd2, g);
     const float temp2 = xsqrt(xsub(1.0f, xmul(temp2_, temp2_)));
-    const f3 v = mk(xmul(sppm_fsin(temp1), temp2), temp2_, xmul(sppm_fcos(temp1), temp2));
+    float sn, cs;
+    fsincos(temp1, sn, cs);
+    const f3 v = mk(xmul(sn, temp2), temp2_, xmul(cs, temp2));
     f3 result = normalize(onb(v, r));
     if (dot(result, n) < 0.0f) result = reflect(result, n);
     return result;
@@ -719,7 +721,9 @@ __device__ __forceinline__ bool eye_path(const JobDesc& J, const JobState* st, u
         const f3 fp = add(CP, scl(rdir, J.focal));
         const float radius = xmul(xsqrt(gpu_rnd(rndv)), J.aperture);
         const float theta = xmul(6.283184f, gpu_rnd(rndv));
-        const f3 lens = add(CP, scl(add(scl(U, sppm_fcos(theta)), scl(V, sppm_fsin(theta))), radius));
+        float sn, cs;
+        fsincos(theta, sn, cs);
+        const f3 lens = add(CP, scl(add(scl(U, cs), scl(V, sn)), radius));
         rdir = normalize(sub(fp, lens));
         rorg = lens;
     }
@@ -1046,7 +1050,9 @@ __device__ __forceinline__ void light_sample(const JobDesc& J, float4& rndv, f3&
 __device__ __forceinline__ f3 cosine_lobe(float4& rndv, f3 n) {
     const float r0 = xmul(6.283184f, gpu_rnd(rndv));
     const float r1 = xsqrt(gpu_rnd(rndv));
-    return onb(mk(xmul(sppm_fsin(r0), r1), xsqrt(xsub(1.0f, xmul(r1, r1))), xmul(sppm_fcos(r0), r1)), n);
+    float sn, cs;
+    fsincos(r0, sn, cs);
+    return onb(mk(xmul(sn, r1), xsqrt(xsub(1.0f, xmul(r1, r1))), xmul(cs, r1)), n);
 }
 
 __device__ __forceinline__ void ibl_sample(const JobDesc& J, float4& rndv, f3& flux, f3& dir, f3& org) {
