@@ -1335,14 +1335,21 @@ __global__ void __launch_bounds__(128) k_photon(LaunchSet ls) {
 //
 // The block's slots are first reordered so that the emissions (a photon with no previous hit or
 // at the bounce limit) come before the bounces: each warp then runs one of the two paths (the
-// state written is per slot, so the order of work changes nothing).
+// state written is per slot, so the order of work changes nothing).  Only the 8-byte hit decides
+// the order, so only it goes through shared memory: the rest of the record is read by the lane that
+// works on it (within the block's lines; an emission reads none of it but the generator).
+//
+// Bound by the instructions of the two paths and the latency of these loads: 10 blocks per SM (48
+// registers).  Us a pass against the whole record staged through shared memory at 9 blocks (56
+// registers) -> this: the Cornell box at 1024^2 297.1 -> 290.8, sixteen jobs 1013 -> 1002, glass and
+// glossy spheres with 517x389 photons 163.9 -> 159.4, a 1M-triangle mesh with 2^21 photons 1039 -> 1036.
+// Blocks of 64 threads (twice the adds to the queue's counter): 297.5, 1024, 162.7, 1059 where
+// these read 293.2, 1008, 160.3, 1046; of 512: 306, 1035, 159.6, 1043.
 template <bool TEX>
-__global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
-    // the slot and its record in processing order (the loads of every slot's record are issued
-    // together, before the reorder)
+__global__ void __launch_bounds__(128, TEX ? 5 : 10) k_photon_gen(LaunchSet ls, RayQueue q) {
+    // the slots and their previous hits in processing order
     __shared__ uint32_t order[128];
     __shared__ int2 rec_hit[128];
-    __shared__ float4 rec_pos[128], rec_flux[128], rec_dir[128], rec_rng[128];
     __shared__ uint32_t warp_emit[4], warp_valid[4], warp_rays[4], block_base;
     __shared__ int block_job;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1351,7 +1358,6 @@ __global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
         const bool valid = g0 < ls.total;
         bool emit = false;
         int2 h = make_int2(-1, 0);
-        float4 pp, pf, pd, rn;
         if (valid) {
             const int k0 = find_job(ls, g0);
             if (threadIdx.x == 0) block_job = k0;
@@ -1359,10 +1365,6 @@ __global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
             const JobState* st0 = J0.state;
             const uint32_t s0 = g0 - first_item(ls, k0);
             if (st0->frame != 0) h = J0.ph.hit[s0];
-            pp = J0.ph.pos[s0];
-            pf = J0.ph.flux[s0];
-            pd = J0.ph.dir[s0];
-            rn = J0.ph.rng[s0];
             emit = h.x < 0 || xadd((float)h.y, 1.0f) >= (float)J0.max_path;
         }
         const unsigned em = __ballot_sync(0xFFFFFFFFu, emit), vm = __ballot_sync(0xFFFFFFFFu, valid);
@@ -1386,10 +1388,6 @@ __global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
                                       : e_total + (v_before - e_before) + __popc(vm & ~em & below);
             order[dst] = g0;
             rec_hit[dst] = h;
-            rec_pos[dst] = pp;
-            rec_flux[dst] = pf;
-            rec_dir[dst] = pd;
-            rec_rng[dst] = rn;
         }
         __syncthreads();
     }
@@ -1410,8 +1408,8 @@ __global__ void __launch_bounds__(128) k_photon_gen(LaunchSet ls, RayQueue q) {
     uint32_t bin = 0, rank = 0;
     if (on) {
         const uint32_t sidx = g - first_item(ls, k);
-        float4 rndv = rec_rng[t];
-        R = photon_generate<TEX>(J, rec_hit[t], rec_pos[t], rec_flux[t], rec_dir[t], rndv, err);
+        float4 rndv = J.ph.rng[sidx];
+        R = photon_generate<TEX>(J, rec_hit[t], J.ph.pos[sidx], J.ph.flux[sidx], J.ph.dir[sidx], rndv, err);
         J.ph.rng[sidx] = rndv;
         if (R.cont) {
             J.ph.flux[sidx] = f4(R.flux, 0.0f);  // flux before the segment, read back by k_photon_store
