@@ -41,8 +41,9 @@ void launch_cell_bounds(const JobDesc* jobs, const uint32_t* job_ids, uint32_t n
 void launch_photon_fp32(const LaunchSet& ls, bool count_traversal, bool textured, cudaStream_t s);
 void launch_photon_gen_fp32(const LaunchSet& ls, const RayQueue& q, bool textured, cudaStream_t s);
 void launch_queue_reset(const RayQueue& q, cudaStream_t s);
+// ahead: the walk that loads a step ahead, for launches of up to kTraceAheadSlots
 void launch_trace_photons_fp32(const LaunchSet& ls, const RayQueue& q, bool count_traversal,
-                               uint32_t persistent_blocks, cudaStream_t s);
+                               uint32_t persistent_blocks, bool ahead, cudaStream_t s);
 void launch_ray_bins(const RayQueue& q, cudaStream_t s);
 // the bins' traversal order from the walks traced since the last call (longest mean first)
 void launch_ray_bins_order(const RayQueue& q, cudaStream_t s);
@@ -50,7 +51,7 @@ void launch_trace_photons_coop(const LaunchSet& ls, const RayQueue& q, bool coun
 // grid_shift: the counting-sort grid's cell split (log2) for jobs with SPPM_FLAG_PHOTON_GRID
 void launch_photon_store_fp32(const LaunchSet& ls, const RayQueue& q, uint32_t block, uint32_t grid_shift,
                               cudaStream_t s);
-uint32_t trace_photons_blocks_per_sm();
+uint32_t trace_photons_blocks_per_sm(bool ahead);
 
 // mixed-precision path (kernels_mixed.cu)
 void launch_trace_photons4(const LaunchSet& ls, const RayQueue& q, uint32_t persistent_blocks, cudaStream_t s);

@@ -1626,8 +1626,11 @@ __global__ void __launch_bounds__(256) k_ray_bins_scatter(RayQueue q) {
 // a 1M-triangle mesh (2^21), 610 -> 568 over 16 jobs.  With fewer rays than lanes the longest walk
 // decides, and what its step waits for: spread over the warps, 2^14 rays take 51 us instead of 70,
 // 2^16 63 instead of 74.
-template <bool COUNT>
-__global__ void __launch_bounds__(128, 9) k_trace_photons(LaunchSet ls, RayQueue q) {
+// AHEAD (launches of up to kTraceAheadSlots): a step loads both nodes that the next one may need before
+// it tests its own box, so the chain of a walk holds the loads alone and not the test between them; twice
+// the loads and 80 registers (6 blocks per SM) that larger launches have no room for.
+template <bool COUNT, bool AHEAD>
+__global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet ls, RayQueue q) {
     const uint32_t total = q.counters[0];
     const int refill = q.refill_steps ? (int)q.refill_steps : 32;
     const unsigned lane = threadIdx.x & 31;
@@ -1729,10 +1732,19 @@ __global__ void __launch_bounds__(128, 9) k_trace_photons(LaunchSet ls, RayQueue
         if (idx >= kDone) continue;
         bool finished = false;
         int it = 0;
+        unsigned long long lo, hi, near_far, links;
+        if (AHEAD) ldg32q(nodes + node, lo, hi, near_far, links);
 #pragma unroll 1
         do {
-            unsigned long long lo, hi, near_far, links;
-            ldg32q(nodes + node, lo, hi, near_far, links);
+            unsigned long long next_lo, next_hi, next_near_far, next_links;  // the node after a hit
+            unsigned long long miss_lo, miss_hi, miss_near_far, miss_links;  // and after a miss
+            if (AHEAD) {
+                const uint32_t last = (uint32_t)nn - 1u;  // (past the end: a node, not used)
+                ldg32q(nodes + min((uint32_t)node + 1u, last), next_lo, next_hi, next_near_far, next_links);
+                ldg32q(nodes + min((uint32_t)node_miss(links), last), miss_lo, miss_hi, miss_near_far, miss_links);
+            } else {
+                ldg32q(nodes + node, lo, hi, near_far, links);
+            }
             if (COUNT) tc.nodes++;
             float tmin, tmax;
             slab_x<true>(R, lo, hi, near_far, tmin, tmax);
@@ -1768,6 +1780,12 @@ __global__ void __launch_bounds__(128, 9) k_trace_photons(LaunchSet ls, RayQueue
                 }
             }
             node = hit ? node + 1 : node_miss(links);
+            if (AHEAD) {
+                lo = hit ? next_lo : miss_lo;
+                hi = hit ? next_hi : miss_hi;
+                near_far = hit ? next_near_far : miss_near_far;
+                links = hit ? next_links : miss_links;
+            }
             it++;
             finished = (uint32_t)node >= (uint32_t)nn;
         } while (!finished && it < refill);
@@ -2222,10 +2240,11 @@ void launch_ray_bins(const RayQueue& q, cudaStream_t s) {
 }
 
 void launch_trace_photons_fp32(const LaunchSet& ls, const RayQueue& q, bool count, uint32_t persistent_blocks,
-                               cudaStream_t s) {
+                               bool ahead, cudaStream_t s) {
     if (!ls.total) return;
-    if (count) k_trace_photons<true><<<persistent_blocks, 128, 0, s>>>(ls, q);
-    else k_trace_photons<false><<<persistent_blocks, 128, 0, s>>>(ls, q);
+    if (count) k_trace_photons<true, false><<<persistent_blocks, 128, 0, s>>>(ls, q);
+    else if (ahead) k_trace_photons<false, true><<<persistent_blocks, 128, 0, s>>>(ls, q);
+    else k_trace_photons<false, false><<<persistent_blocks, 128, 0, s>>>(ls, q);
     if (q.tail_lanes && q.tail_list) {
         // one warp per handed-over walk: enough warps for every SM
         if (count) k_trace_photons_tail<true><<<persistent_blocks, 128, 0, s>>>(ls, q);
@@ -2245,10 +2264,14 @@ void launch_photon_store_fp32(const LaunchSet& ls, const RayQueue& q, uint32_t b
     if (ls.total) k_photon_store<<<blocks_for(q.capacity, b), b, 0, s>>>(ls, q, grid_shift);
 }
 
-uint32_t trace_photons_blocks_per_sm() {
+template <bool AHEAD>
+static uint32_t trace_photons_fit() {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_trace_photons<false>, 128, 0) != cudaSuccess) n = 4;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_trace_photons<false, AHEAD>, 128, 0) != cudaSuccess) n = 4;
     return n > 0 ? (uint32_t)n : 1u;
+}
+uint32_t trace_photons_blocks_per_sm(bool ahead) {
+    return ahead ? trace_photons_fit<true>() : trace_photons_fit<false>();
 }
 void launch_gather_fp32(const LaunchSet& ls, uint32_t block, cudaStream_t s) {
     const uint32_t b = block_or(block, 256);

@@ -254,6 +254,7 @@ struct Runner {
     bool fp64_stats = false;       // some active job keeps IEEE double statistics
     bool wide_ok = false;          // every active job has the 4-wide BVH (the plain path may use it)
     uint32_t trace_fit4 = 0;       // 4-wide traversal blocks of 128 threads that fit on one SM
+    uint32_t trace_fit_ahead = 0;  // and blocks of the walk that loads a step ahead
     std::vector<StageEvent> pending;
     size_t open_stage[SPPM_STAGE_COUNT] = {0};  // pending entry of each stage's last start
     std::vector<cudaEvent_t> event_pool;
