@@ -64,7 +64,11 @@ struct TraversalCount {
     uint32_t nodes = 0, tris = 0;
 };
 
-template <bool PHOTON, bool COUNT = false>
+// The walk of one ray by one thread.  The divisions of the triangle test (tri_test_exact) follow one
+// another's tests, as few lanes need all three, and the loop ends in one place, so that a warp's lanes
+// meet before the next node (u > 1 leaves w < 0 whatever v is).  AHEAD: both nodes that may come next
+// are loaded before this one is tested (k_trace_photons).
+template <bool PHOTON, bool COUNT = false, bool AHEAD = false>
 __device__ __forceinline__ Hit trace_exact(const DevScene& s, f3 org, f3 dir, bool cull, uint32_t& err,
                                            TraversalCount* cnt = nullptr) {
     Hit h;
@@ -77,13 +81,18 @@ __device__ __forceinline__ Hit trace_exact(const DevScene& s, f3 org, f3 dir, bo
     const RayX R = ray_x(org, dir, face);
     const int32_t nn = (int32_t)s.num_nodes;
     int32_t i = 0;
-    for (int32_t steps = 0;; steps++) {
-        if (steps > nn) {
-            err |= kErrWatchdogTraverse;
-            break;
+    unsigned long long lo, hi, near_far, links;
+    if (AHEAD) ldg32q(nodes, lo, hi, near_far, links);
+    int32_t steps = 0;
+    do {
+        unsigned long long next_lo, next_hi, next_near_far, next_links, miss_lo, miss_hi, miss_near_far, miss_links;
+        if (AHEAD) {
+            const uint32_t last = (uint32_t)nn - 1u;
+            ldg32q(nodes + min((uint32_t)i + 1u, last), next_lo, next_hi, next_near_far, next_links);
+            ldg32q(nodes + min((uint32_t)node_miss(links), last), miss_lo, miss_hi, miss_near_far, miss_links);
+        } else {
+            ldg32q(nodes + i, lo, hi, near_far, links);
         }
-        unsigned long long lo, hi, near_far, links;
-        ldg32q(nodes + i, lo, hi, near_far, links);
         if (COUNT) cnt->nodes++;
         float tmin, tmax;
         slab_x<false>(R, lo, hi, near_far, tmin, tmax);
@@ -95,20 +104,38 @@ __device__ __forceinline__ Hit trace_exact(const DevScene& s, f3 org, f3 dir, bo
             const float4 a = __ldg(&s.tri_isect[(size_t)t * 3 + 0]);
             const float4 b = __ldg(&s.tri_isect[(size_t)t * 3 + 1]);
             const float4 c = __ldg(&s.tri_isect[(size_t)t * 3 + 2]);
-            float tt, u, v, w;
-            if (tri_test_exact(a, b, c, org, dir, !PHOTON && cull, h.t, tt, u, v, w)) {
-                h.t = tt;
-                h.tri = t;
-                h.mat = __float_as_int(c.y);
-                h.bu = v;
-                h.bv = w;
-                h.bw = u;
+            const f3 e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, c.x);
+            const f3 pv = cross(dir, e1);
+            const float det = dot(e0, pv);
+            const f3 tv = sub(org, mk(a.x, a.y, a.z));
+            const f3 qv = cross(tv, e0);
+            const float u = xdiv(dot(tv, pv), det);
+            if (u >= 0.0f && u <= 1.0f && (PHOTON || !cull || det > 1e-10f)) {
+                const float v = xdiv(dot(dir, qv), det);
+                const float w = xsub(xsub(1.0f, u), v);
+                if (v >= 0.0f && w >= 0.0f) {
+                    const float tt = xdiv(dot(e1, qv), det);
+                    if (tt >= 0.0f && tt < h.t) {
+                        h.t = tt;
+                        h.tri = t;
+                        h.mat = __float_as_int(c.y);
+                        h.bu = v;
+                        h.bv = w;
+                        h.bw = u;
+                    }
+                }
             }
         }
-        const int32_t next = hit ? i + 1 : node_miss(links);
-        if (next < 0 || next >= nn) break;
-        i = next;
-    }
+        i = hit ? i + 1 : node_miss(links);
+        if (AHEAD) {
+            lo = hit ? next_lo : miss_lo;
+            hi = hit ? next_hi : miss_hi;
+            near_far = hit ? next_near_far : miss_near_far;
+            links = hit ? next_links : miss_links;
+        }
+        steps++;
+    } while ((uint32_t)i < (uint32_t)nn && steps <= nn);
+    if ((uint32_t)i < (uint32_t)nn) err |= kErrWatchdogTraverse;
     return h;
 }
 
@@ -850,8 +877,13 @@ __device__ __forceinline__ bool tile_pixel(const JobDesc& J, uint32_t item, uint
 // sixteen 512^2 frames 1043 -> 1029, the Cornell box at 1024^2 302 -> 301; and 8 resident blocks
 // (64 registers, 12 bytes spilled) 1049 -> 1044, 1029 -> 1025, 301 -> 301.  The textured path needs more
 // registers than that.
-template <bool MIXED, bool TEX>
-__global__ void __launch_bounds__(128, TEX ? 5 : 8)
+// AHEAD (launches of up to kEyeAheadItems, untextured): with few warps the paths' chains decide.  Us a pass
+// without / with it, 512^2 photons: glass and glossy spheres 166.8 / 157.6 at 256^2 pixels, 173.2 / 167.4
+// at 512^2, 196.9 / 194.3 at 1024x768; Cornell box 121.9 / 121.4, 125.7 / 126.0, 148.3 / 149.7; 102k-triangle
+// mesh 180.8 / 179.3, 189.6 / 190.1, 213.7 / 217.6; 1M triangles 337.2 / 330.8, 343.7 / 338.3, 367.5 / 367.6.
+constexpr uint32_t kEyeAheadItems = 1u << 18;
+template <bool MIXED, bool TEX, bool AHEAD = false>
+__global__ void __launch_bounds__(128, TEX ? 5 : AHEAD ? 6 : 8)
     k_eye(LaunchSet ls, uint32_t* deferred_n, uint32_t* deferred, uint32_t deferred_cap) {
     // the block's segment count for the job of its first item: one global add per block, made by the
     // last of its threads to get there (no barrier: the others' registers are free when their paths
@@ -879,7 +911,7 @@ __global__ void __launch_bounds__(128, TEX ? 5 : 8)
                 return false;
             }
         }
-        h = trace_exact<false>(J.scene, org, dir, cull, err);
+        h = trace_exact<false, false, AHEAD>(J.scene, org, dir, cull, err);
         return true;
     }, o);
     if (done) eye_write(J, st, p, o);
@@ -2197,7 +2229,10 @@ static void launch_eye_t(const LaunchSet& ls, const RayQueue& q, bool mixed, uin
         k_eye<true, TEX><<<blocks_for(ls.total, b), b, 0, s>>>(ls, nullptr, nullptr, 0);
         return;
     }
-    k_eye<false, TEX><<<blocks_for(ls.total, b), b, 0, s>>>(ls, q.counters + 3, q.eye_deferred, kEyeDeferred);
+    if (!TEX && ls.total <= kEyeAheadItems)
+        k_eye<false, false, true><<<blocks_for(ls.total, b), b, 0, s>>>(ls, q.counters + 3, q.eye_deferred, kEyeDeferred);
+    else
+        k_eye<false, TEX><<<blocks_for(ls.total, b), b, 0, s>>>(ls, q.counters + 3, q.eye_deferred, kEyeDeferred);
     // a fixed grid (the count is on the device): blocks beyond the deferred pixels exit at once
     k_eye_coop<TEX><<<32, kBlockWalk, 0, s>>>(ls, q.counters + 3, q.eye_deferred, kEyeDeferred);
 }
