@@ -378,19 +378,29 @@ __device__ __forceinline__ void grid_accumulate(const PhotonGrid& grid, uint32_t
 // box), the warp walks that union together: a lane per cell looks up the cells' record ranges in
 // one round, a warp scan concatenates them, and the concatenated records are loaded and decoded in
 // batches of 32 (a lane per record, the test that the record lies in its cell included) into
-// shared memory, where every lane tests every record of the batch against its own hit point.  A
+// shared memory -- direction and fixed-point flux too, once per record and not per pixel that takes it --
+// where every lane tests every record of the batch against its own hit point.  A
 // lane accepts exactly the photons inside its radius (the union holds all of them, and each photon
 // sits in one cell), so its sums equal its own walk's; otherwise every lane walks its own cells
 // (grid_accumulate).  All 32 lanes call it.
+//
+// Bound by the instructions of the tests and of the accepted records, which some lane of the warp takes
+// nearly always, and by tiles of uneven photon counts: 1.05M pixels of the Cornell box with 2^20 photons
+// 181 us with every pixel decoding what it takes, in blocks of 256 threads; 157 decoded once; 150 with
+// 5 such blocks per SM for 4; 142 in blocks of 128, whose tiles wait for fewer others (64: 142, 32: 148).
 constexpr uint32_t kCoopMaxCells = 128;
+constexpr uint32_t kGridGatherBlock = 128;  // threads (at most) of the grid gather's blocks
 
 struct GridWarpSmem {
     // the union's cells that hold records, in walk order
     uint32_t cell_off[kCoopMaxCells + 1];  // first index in the concatenation of their records
     uint32_t cell_beg[kCoopMaxCells];      // first record
     uint32_t cell_x[kCoopMaxCells], cell_y[kCoopMaxCells], cell_z[kCoopMaxCells];  // coordinates
-    float4 rec[32];                        // the batch: the position (cells' fixed point) + flux r|g
-    uint32_t w[32];                        // flux b | direction
+    // the batch, decoded: the position (cells' fixed point) and the direction's x; its y and z; the flux
+    float4 rec[32];
+    float2 dir[32];
+    ulonglong2 rg[32];
+    unsigned long long b[32];
 };
 
 __device__ __forceinline__ void grid_gather_warp(const LaunchSet& ls, const uint32_t* slot_prefix,
@@ -536,8 +546,13 @@ __device__ __forceinline__ void grid_gather_warp(const LaunchSet& ls, const uint
         const unsigned kept = __ballot_sync(full, keep);
         if (keep) {
             const uint32_t at = __popc(kept & ((1u << lane) - 1u));
+            const uint32_t rz = __float_as_uint(ent.w);
+            float2 yz;
+            grid_oct8_decode(w >> 16, ent.w, yz.x, yz.y);
             sm.rec[at] = ent;
-            sm.w[at] = w;
+            sm.dir[at] = yz;
+            sm.rg[at] = make_ulonglong2(grid_half_fixed(rz & 0xFFFFu), grid_half_fixed(rz >> 16));
+            sm.b[at] = grid_half_fixed(w & 0xFFFFu);
         }
         __syncwarp();
         const uint32_t n = __popc(kept);
@@ -548,12 +563,12 @@ __device__ __forceinline__ void grid_gather_warp(const LaunchSet& ls, const uint
                 const float dx = __fsub_rn(c.x, vx), dy = __fsub_rn(c.y, vy), dz = __fsub_rn(c.z, vz);
                 const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
                 if (!(d2 < rq2)) continue;
-                const uint32_t ww = sm.w[j];
-                if (!(grid_oct8_dot(ww >> 16, qn4.x, qn4.y, qn4.z) < 0.0f)) continue;
-                const uint32_t rz = __float_as_uint(c.w);
-                sr += grid_half_fixed(rz & 0xFFFFu);
-                sg += grid_half_fixed(rz >> 16);
-                sb += grid_half_fixed(ww & 0xFFFFu);
+                const float2 yz = sm.dir[j];
+                if (!(grid_dir_dot(c.w, yz.x, yz.y, qn4.x, qn4.y, qn4.z) < 0.0f)) continue;
+                const ulonglong2 rg = sm.rg[j];
+                sr += rg.x;
+                sg += rg.y;
+                sb += sm.b[j];
                 m++;
             }
         }
@@ -570,7 +585,8 @@ __device__ __forceinline__ void grid_gather_warp(const LaunchSet& ls, const uint
 // launched when some job of the launch keeps IEEE double statistics; ANY_GRID: when some job uses
 // the grid; slot_prefix: the hash-slot launch set's prefix sums)
 template <bool ANY_F64, bool ANY_GRID>
-__global__ void __launch_bounds__(256) k_gather_mixed(LaunchSet ls, const uint32_t* slot_prefix, PhotonGrid grid) {
+__global__ void __launch_bounds__(ANY_GRID ? kGridGatherBlock : 256, ANY_GRID && !ANY_F64 ? 10 : 1)
+    k_gather_mixed(LaunchSet ls, const uint32_t* slot_prefix, PhotonGrid grid) {
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     bool live = gi < ls.total;
     int k = 0;
@@ -589,7 +605,7 @@ __global__ void __launch_bounds__(256) k_gather_mixed(LaunchSet ls, const uint32
     }
     float gfx = 0.0f, gfy = 0.0f, gfz = 0.0f, gM = 0.0f;
     if (ANY_GRID) {
-        __shared__ GridWarpSmem s_grid[256 / 32];
+        __shared__ GridWarpSmem s_grid[kGridGatherBlock / 32];
         grid_gather_warp(ls, slot_prefix, grid, live, (uint32_t)k, p, s_grid[threadIdx.x >> 5], gfx, gfy, gfz, gM);
     }
     if (!live) return;
@@ -747,7 +763,8 @@ void launch_slot_fill(const LaunchSet& hash_slots, cudaStream_t s) {
 }
 void launch_gather_mixed(const LaunchSet& ls, uint32_t block, bool any_fp64, const uint32_t* slot_prefix,
                          const PhotonGrid* grid, cudaStream_t s) {
-    const uint32_t b = block >= 32 && block <= 256 && block % 32 == 0 ? block : 256;
+    const uint32_t most = grid ? kGridGatherBlock : 256;
+    const uint32_t b = block >= 32 && block <= 256 && block % 32 == 0 ? (block < most ? block : most) : most;
     if (!ls.total) return;
     const PhotonGrid g = grid ? *grid : PhotonGrid{};
     const uint32_t n = blocks_for(ls.total, b);

@@ -77,18 +77,26 @@ __device__ __forceinline__ uint32_t grid_oct8(float x, float y, float z) {
     return ((uint32_t)a & 0xFFu) | (((uint32_t)b & 0xFFu) << 8);
 }
 
-// dot(n, d) for the (unnormalised) direction d an octahedral code stands for: its sign is what
-// the gather's facing test reads; the decoded components are small integers (exact)
-__device__ __forceinline__ float grid_oct8_dot(uint32_t code, float nx, float ny, float nz) {
-    float x = (float)(int)(int8_t)(code & 0xFFu), y = (float)(int)(int8_t)((code >> 8) & 0xFFu);
+// the (unnormalised) direction an octahedral code stands for; the components are small integers (exact)
+__device__ __forceinline__ void grid_oct8_decode(uint32_t code, float& x, float& y, float& z) {
+    x = (float)(int)(int8_t)(code & 0xFFu), y = (float)(int)(int8_t)((code >> 8) & 0xFFu);
     const float ax = fabsf(x), ay = fabsf(y);
-    const float z = 127.0f - ax - ay;
+    z = 127.0f - ax - ay;
     if (z < 0.0f) {
         const float tx = (127.0f - ay) * copysignf(1.0f, x);
         y = (127.0f - ax) * copysignf(1.0f, y);
         x = tx;
     }
+}
+
+// dot(n, d) for such a direction: its sign is what the gather's facing test reads
+__device__ __forceinline__ float grid_dir_dot(float x, float y, float z, float nx, float ny, float nz) {
     return __fadd_rn(__fadd_rn(__fmul_rn(nx, x), __fmul_rn(ny, y)), __fmul_rn(nz, z));
+}
+__device__ __forceinline__ float grid_oct8_dot(uint32_t code, float nx, float ny, float nz) {
+    float x, y, z;
+    grid_oct8_decode(code, x, y, z);
+    return grid_dir_dot(x, y, z, nx, ny, nz);
 }
 
 __device__ __forceinline__ uint32_t grid_half(float v) {

@@ -346,7 +346,8 @@ typedef struct sppm_tuning {
                                      on the mixed path's rays in queue order)                   */
     uint32_t eye_block;           /* threads per block of the eye pass (0 = 128; 32..128)       */
     uint32_t store_block;         /* of the photon store + hash insertion (0 = 128; 32..128)    */
-    uint32_t gather_block;        /* of the gather + progressive update (0 = 256; 32..256)      */
+    uint32_t gather_block;        /* of the gather + progressive update (0 = 256; 32..256; of the
+                                     counting-sort grid at most 128)                            */
     uint32_t unbinned_rays;       /* 1: photon rays traced in queue order instead of binned.  Until
                                      shapes are set the library chooses (and reports 0): bins for
                                      the plain path's single job with 3/4 * 2^20 photon slots or
