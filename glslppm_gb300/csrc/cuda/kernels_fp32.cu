@@ -1928,7 +1928,13 @@ __global__ void __launch_bounds__(128) k_photon_store(LaunchSet ls, RayQueue q, 
 // loads -- pixel state, the eight cells' winners, their photons -- at 32 warps per SM (64 registers);
 // the bounds of the in-cell test are nine planes per pixel, loaded once, not six per cell: 57.8 -> 52.1
 // us on the Cornell box (1024^2), 189 -> 171 over 16 jobs.
-__global__ void __launch_bounds__(256, 4) k_gather(LaunchSet ls) {
+// BLOCKS per SM: 5 (48 registers, 52 bytes spilled) where a launch has waves of blocks to fill them.  Us a
+// pass with 1024x512 photons, 4 / 5 blocks: Cornell box 168.1 / 171.4 at 512^2 pixels, 186.9 / 189.2 at
+// 768^2, 210.1 / 209.2 at 1024^2, 216.2 / 214.7 at 1280x1024, 343.8 / 332.9 at 2048^2; 102k-triangle mesh
+// 256.3 / 254.8, 269.0 / 268.9, 288.5 / 285.7, 297.5 / 295.2, 407.0 / 397.5; sixteen jobs 978 / 968.
+constexpr uint32_t kGatherWideItems = 1u << 20;
+template <int BLOCKS>
+__global__ void __launch_bounds__(256, BLOCKS) k_gather(LaunchSet ls) {
     const uint32_t g = grid_tid();
     if (g >= ls.total) return;
     const int k = find_job(ls, g);
@@ -2310,7 +2316,8 @@ uint32_t trace_photons_blocks_per_sm(bool ahead) {
 }
 void launch_gather_fp32(const LaunchSet& ls, uint32_t block, cudaStream_t s) {
     const uint32_t b = block_or(block, 256);
-    if (ls.total) k_gather<<<blocks_for(ls.total, b), b, 0, s>>>(ls);
+    if (ls.total >= kGatherWideItems) k_gather<5><<<blocks_for(ls.total, b), b, 0, s>>>(ls);
+    else if (ls.total) k_gather<4><<<blocks_for(ls.total, b), b, 0, s>>>(ls);
 }
 void launch_resolve_fp32(const LaunchSet& ls, uint32_t display, cudaStream_t s) {
     if (ls.total) k_resolve<<<blocks_for(ls.total, 256), 256, 0, s>>>(ls, display);
