@@ -4,8 +4,8 @@
 // pixels into a ping-pong texture; each output texel applies min.fs / max.fs / sum.fs to the four
 // texels (i,j), (i+n,j), (i,j+n), (i+n,j+n) of the previous level, and the host reads texel (0,0).
 // The folds of consecutive levels of one output texel read inputs that no other output reads, so a
-// launch does up to three levels (64 input texels a thread, no texel written between) until 128 x 128
-// texels are left, which one block folds to the end.  The sums are evaluated as ((v0 + v1) + v2) + v3
+// launch does up to four levels (no texel written between) until at most 128 x 128 texels are left,
+// which one block folds to the end.  The sums are evaluated as ((v0 + v1) + v2) + v3
 // with non-fused adds in the reference's order, so all three results are bit-identical to its fold.
 //
 // 1024 x 1024 (16 MiB): two launches instead of ten, and a scratch kept between calls: 249 -> 36 us a
@@ -57,6 +57,30 @@ __global__ void __launch_bounds__(128) k_reduce_levels(const float4* src, uint32
     dst[(size_t)j * dst_stride + i] = fold_levels<OP, K>(src, src_stride, i, j, n);
 }
 
+// Four levels, 256 input texels an output: a block folds 32 outputs, each of its 16 warps two levels of
+// one sixteenth of their inputs (16 loads a thread, all of a 1024 x 1024 texture in flight at once), and
+// the last two levels through shared memory.  In place as above: a block reads its own output texels
+// before the barrier and writes them after it.  64 texels a thread, three levels without shared
+// memory, took 12.4 us for 1024 x 1024 (16 MiB) and left four times the texels for the one block of the
+// tail, 6.0 us; this 6.7 and 4.2.
+template <int OP>
+__global__ void __launch_bounds__(512) k_reduce_levels4(const float4* src, uint32_t src_stride, float4* dst,
+                                                      uint32_t dst_stride, uint32_t n) {
+    __shared__ float4 s[16][32];
+    const uint32_t lane = threadIdx.x & 31u, q1 = threadIdx.x >> 7, q2 = (threadIdx.x >> 5) & 3u;
+    const uint32_t t = blockIdx.x * 32 + lane, i = t % n, j = t / n;
+    if (t < n * n)
+        s[threadIdx.x >> 5][lane] =
+            fold_levels<OP, 2>(src, src_stride, i + (q1 & 1u) * n + (q2 & 1u) * 2 * n,
+                               j + (q1 >> 1) * n + (q2 >> 1) * 2 * n, 4 * n);
+    __syncthreads();
+    if (t < n * n && q2 == 0)
+        s[threadIdx.x >> 5][lane] = fold4<OP>(s[4 * q1][lane], s[4 * q1 + 1][lane], s[4 * q1 + 2][lane], s[4 * q1 + 3][lane]);
+    __syncthreads();
+    if (t < n * n && threadIdx.x < 32)
+        dst[(size_t)j * dst_stride + i] = fold4<OP>(s[0][lane], s[4][lane], s[8][lane], s[12][lane]);
+}
+
 // the last levels in one block: n x n texels (n <= kReduceTail) to one.  A thread folds up to two
 // levels from memory, the rest go through shared memory.
 constexpr uint32_t kReduceTail = 128;
@@ -85,9 +109,9 @@ template <int OP>
 static void reduce_op(const float4* src, uint32_t n, float4* scratch, cudaStream_t s) {
     uint32_t stride = n;
     while (n > kReduceTail) {
-        const uint32_t k = n >= 8 * kReduceTail ? 3 : (n == 4 * kReduceTail ? 2 : 1), m = n >> k;
+        const uint32_t k = n >= 8 * kReduceTail ? 4 : (n == 4 * kReduceTail ? 2 : 1), m = n >> k;
         const uint32_t out_stride = src == scratch ? stride : m, blocks = (m * m + 127) / 128;
-        if (k == 3) k_reduce_levels<OP, 3><<<blocks, 128, 0, s>>>(src, stride, scratch, out_stride, m);
+        if (k == 4) k_reduce_levels4<OP><<<(m * m + 31) / 32, 512, 0, s>>>(src, stride, scratch, out_stride, m);
         else if (k == 2) k_reduce_levels<OP, 2><<<blocks, 128, 0, s>>>(src, stride, scratch, out_stride, m);
         else k_reduce_levels<OP, 1><<<blocks, 128, 0, s>>>(src, stride, scratch, out_stride, m);
         src = scratch;
@@ -100,7 +124,7 @@ static void reduce_op(const float4* src, uint32_t n, float4* scratch, cudaStream
 // texels of scratch: the first launch's output, at least the result's
 size_t reduce_scratch_texels(uint32_t resolution) {
     if (resolution <= kReduceTail) return 1;
-    const size_t m = resolution >= 8 * kReduceTail ? resolution / 8 : kReduceTail;
+    const size_t m = resolution >= 8 * kReduceTail ? resolution / 16 : kReduceTail;
     return m * m;
 }
 
