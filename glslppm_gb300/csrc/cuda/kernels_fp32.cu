@@ -882,8 +882,14 @@ __device__ __forceinline__ bool tile_pixel(const JobDesc& J, uint32_t item, uint
 // at 512^2, 196.9 / 194.3 at 1024x768; Cornell box 121.9 / 121.4, 125.7 / 126.0, 148.3 / 149.7; 102k-triangle
 // mesh 180.8 / 179.3, 189.6 / 190.1, 213.7 / 217.6; 1M triangles 337.2 / 330.8, 343.7 / 338.3, 367.5 / 367.6.
 constexpr uint32_t kEyeAheadItems = 1u << 18;
+// The mixed path's walk has no such chain to shorten, but at 8 blocks it spills 280 bytes of loads: up to
+// kEyeMixedItems it runs with all 93 registers (5 blocks).  Us a pass, 8 / 5 blocks, 1024x512 photons, an
+// eye pass in ten: glass and glossy spheres 228.9 / 227.1 at 256^2 pixels, 244.7 / 239.3 at 512^2,
+// 252.1 / 248.8 at 640x600, but Cornell box 268.4 / 271.1 and 102k-triangle mesh 327.8 / 332.6 at 1536^2;
+// an eye pass in each, 133x234: 287 / 276.
+constexpr uint32_t kEyeMixedItems = 1u << 19;
 template <bool MIXED, bool TEX, bool AHEAD = false>
-__global__ void __launch_bounds__(128, TEX ? 5 : AHEAD ? 6 : 8)
+__global__ void __launch_bounds__(128, TEX ? 5 : AHEAD ? (MIXED ? 5 : 6) : 8)
     k_eye(LaunchSet ls, uint32_t* deferred_n, uint32_t* deferred, uint32_t deferred_cap) {
     // the block's segment count for the job of its first item: one global add per block, made by the
     // last of its threads to get there (no barrier: the others' registers are free when their paths
@@ -2232,7 +2238,8 @@ template <bool TEX>
 static void launch_eye_t(const LaunchSet& ls, const RayQueue& q, bool mixed, uint32_t block, cudaStream_t s) {
     const uint32_t b = block_or(block, 128);
     if (mixed) {
-        k_eye<true, TEX><<<blocks_for(ls.total, b), b, 0, s>>>(ls, nullptr, nullptr, 0);
+        if (!TEX && ls.total <= kEyeMixedItems) k_eye<true, false, true><<<blocks_for(ls.total, b), b, 0, s>>>(ls, nullptr, nullptr, 0);
+        else k_eye<true, TEX><<<blocks_for(ls.total, b), b, 0, s>>>(ls, nullptr, nullptr, 0);
         return;
     }
     if (!TEX && ls.total <= kEyeAheadItems)

@@ -389,6 +389,11 @@ __device__ __forceinline__ void grid_accumulate(const PhotonGrid& grid, uint32_t
 // 181 us with every pixel decoding what it takes, in blocks of 256 threads; 157 decoded once; 150 with
 // 5 such blocks per SM for 4; 142 in blocks of 128, whose tiles wait for fewer others (64: 142, 32: 148).
 constexpr uint32_t kCoopMaxCells = 128;
+// From this many pixels the blocks are bounded to 48 registers (10 per SM; 64 bytes spilled).  Us a pass with
+// 1024x512 photons, 8 / 10 blocks: Cornell box 235.1 / 240.0 at 640x600 pixels, 250.3 / 252.3 at 768^2,
+// 273.9 / 272.8 at 1024^2, 347 / 337 at 1536^2; glass and glossy spheres 317 / 319, 340.5 / 339.6, 393 / 386,
+// 545 / 529; 102k-triangle mesh 337 / 344, 349 / 354, 381.0 / 382.8, 448 / 446.
+constexpr uint32_t kGridWideItems = 1u << 20;
 constexpr uint32_t kGridGatherBlock = 128;  // threads (at most) of the grid gather's blocks
 
 struct GridWarpSmem {
@@ -584,8 +589,8 @@ __device__ __forceinline__ void grid_gather_warp(const LaunchSet& ls, const uint
 // the counting-sort grid), FP32 flux gathering and double-float statistics (ANY_F64: the variant
 // launched when some job of the launch keeps IEEE double statistics; ANY_GRID: when some job uses
 // the grid; slot_prefix: the hash-slot launch set's prefix sums)
-template <bool ANY_F64, bool ANY_GRID>
-__global__ void __launch_bounds__(ANY_GRID ? kGridGatherBlock : 256, ANY_GRID && !ANY_F64 ? 10 : 1)
+template <bool ANY_F64, bool ANY_GRID, bool WIDE = false>
+__global__ void __launch_bounds__(ANY_GRID ? kGridGatherBlock : 256, WIDE ? 10 : 1)
     k_gather_mixed(LaunchSet ls, const uint32_t* slot_prefix, PhotonGrid grid) {
     const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
     bool live = gi < ls.total;
@@ -770,6 +775,7 @@ void launch_gather_mixed(const LaunchSet& ls, uint32_t block, bool any_fp64, con
     const uint32_t n = blocks_for(ls.total, b);
     if (grid) {
         if (any_fp64) k_gather_mixed<true, true><<<n, b, 0, s>>>(ls, slot_prefix, g);
+        else if (ls.total >= kGridWideItems) k_gather_mixed<false, true, true><<<n, b, 0, s>>>(ls, slot_prefix, g);
         else k_gather_mixed<false, true><<<n, b, 0, s>>>(ls, slot_prefix, g);
     } else {
         if (any_fp64) k_gather_mixed<true, false><<<n, b, 0, s>>>(ls, slot_prefix, g);
