@@ -627,9 +627,30 @@ __device__ __forceinline__ float xorshift_frand(uint32_t* s) {
     return xmul(__uint2float_rn(s[3]), 1.0f / 4294967295.0f);
 }
 
+// (four hash slots and four bins a thread: one search for the job and two wide stores)
+__device__ __forceinline__ void begin_job(const JobDesc& J) {
+    JobState* st = J.state;
+    const uint32_t f = st->frames_started;
+    st->frame = f;
+    st->frames_started = f + 1;
+    st->emitted_frame = 0;
+    st->segments_frame = 0;
+    const uint32_t interval = J.eye_interval ? J.eye_interval : 1u;
+    st->is_eye_frame = (f % interval) == 0;
+    if (st->is_eye_frame) {
+        // AAOffset (glslppm.cpp:276-277)
+        st->aa[0] = xmul(xsub(xorshift_frand(st->xs), 0.5f), 1.25f);
+        st->aa[1] = xmul(xsub(xorshift_frand(st->xs), 0.5f), 1.25f);
+        st->eye_samples += 1;
+        for (int c = 0; c < 3; c++) {
+            st->bbmax_key[c] = 0u;           // below every float
+            st->bbmin_key[c] = 0xFFFFFFFFu;  // above every float
+        }
+    }
+}
 __global__ void k_frame_begin(LaunchSet ls, RayQueue q) {
-    const uint32_t g = grid_tid();
-    if (g == 0 && q.counters) {
+    const uint32_t t = grid_tid();
+    if (t == 0 && q.counters) {
         q.counters[0] = 0;
         q.counters[1] = 0;
         q.counters[2] = 0;
@@ -637,32 +658,26 @@ __global__ void k_frame_begin(LaunchSet ls, RayQueue q) {
         q.counters[4] = 0;
         q.counters[7] += 1u;  // frames since the bins were last reordered
     }
-    if (q.bins && g < kBinCounters * kRayBins) q.bins[g] = 0u;
-    if (g >= ls.total) return;
+    static_assert(kBinCounters * kRayBins % 4 == 0, "bins must split into uint4");
+    if (q.bins && t < kBinCounters * kRayBins / 4) reinterpret_cast<uint4*>(q.bins)[t] = make_uint4(0u, 0u, 0u, 0u);
+    if (t > (ls.total - 1u) / 4u) return;
+    const uint32_t g = 4u * t, n = min(ls.total - g, 4u);
     const int k = find_job(ls, g);
     const JobDesc& J = job_of(ls, k);
     const uint32_t local = g - first_item(ls, k);
-    J.winner[local] = kEmptySlot;
-    J.count[local] = 0;
-    if (local == 0) {
-        JobState* st = J.state;
-        const uint32_t f = st->frames_started;
-        st->frame = f;
-        st->frames_started = f + 1;
-        st->emitted_frame = 0;
-        st->segments_frame = 0;
-        const uint32_t interval = J.eye_interval ? J.eye_interval : 1u;
-        st->is_eye_frame = (f % interval) == 0;
-        if (st->is_eye_frame) {
-            // AAOffset (glslppm.cpp:276-277)
-            st->aa[0] = xmul(xsub(xorshift_frand(st->xs), 0.5f), 1.25f);
-            st->aa[1] = xmul(xsub(xorshift_frand(st->xs), 0.5f), 1.25f);
-            st->eye_samples += 1;
-            for (int c = 0; c < 3; c++) {
-                st->bbmax_key[c] = 0u;           // below every float
-                st->bbmin_key[c] = 0xFFFFFFFFu;  // above every float
-            }
-        }
+    if (n == 4u && local + 4u <= J.hash_num && local % 4u == 0u) {
+        *reinterpret_cast<uint4*>(J.winner + local) = make_uint4(kEmptySlot, kEmptySlot, kEmptySlot, kEmptySlot);
+        *reinterpret_cast<uint4*>(J.count + local) = make_uint4(0u, 0u, 0u, 0u);
+        if (local == 0) begin_job(J);
+        return;
+    }
+    for (uint32_t i = g; i < g + n; i++) {
+        const int ki = find_job(ls, i);
+        const JobDesc& Ji = job_of(ls, ki);
+        const uint32_t li = i - first_item(ls, ki);
+        Ji.winner[li] = kEmptySlot;
+        Ji.count[li] = 0;
+        if (li == 0) begin_job(Ji);
     }
 }
 
@@ -2226,8 +2241,9 @@ void launch_gather_states(const JobDesc* jobs, const StateGather& list, JobState
     if (list.n) k_gather_states<<<list.n, 64, 0, s>>>(jobs, list, out);
 }
 void launch_frame_begin(const LaunchSet& ls, const RayQueue& q, cudaStream_t s) {
-    const uint32_t n = q.bins && ls.total < kBinCounters * kRayBins ? kBinCounters * kRayBins : ls.total;
-    if (ls.total) k_frame_begin<<<blocks_for(n, 256), 256, 0, s>>>(ls, q);
+    if (!ls.total) return;
+    const uint32_t items = (ls.total - 1) / 4 + 1, bins = q.bins ? kBinCounters * kRayBins / 4 : 0;
+    k_frame_begin<<<blocks_for(items > bins ? items : bins, 256), 256, 0, s>>>(ls, q);
 }
 // block sizes: a multiple of 32 up to the kernel's launch bound (0 or anything else: the bound)
 static uint32_t block_or(uint32_t block, uint32_t bound) {
