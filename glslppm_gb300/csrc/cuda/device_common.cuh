@@ -385,8 +385,8 @@ __device__ __forceinline__ int32_t node_tri(unsigned long long links) { return (
 // Moller-Trumbore on the packed operands (a = v0 | e0.x, b = e0.yz | e1.xy, c.x = e1.z), every
 // operation correctly rounded in the shaders' order, so a triangle's t, u, v and w are the same
 // numbers wherever this is called (plain and mixed traversals alike).  Returns true when the
-// triangle is hit at 0 <= t < tbest; cull: reject det <= 1e-10 (back faces of a first eye bounce).
-// tri_hit_exact: the same test without the comparison against the closest hit so far.
+// triangle is hit at t >= 0; cull: reject det <= 1e-10 (back faces of a first eye bounce).  The walks of
+// one ray per thread write it out, each division after the one before has passed.
 __device__ __forceinline__ bool tri_hit_exact(const float4& a, const float4& b, const float4& c, f3 org, f3 dir,
                                               bool cull, float& tt, float& u, float& v, float& w) {
     const f3 v0 = mk(a.x, a.y, a.z), e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, c.x);
@@ -400,10 +400,6 @@ __device__ __forceinline__ bool tri_hit_exact(const float4& a, const float4& b, 
     tt = xdiv(dot(e1, qv), det);
     w = xsub(xsub(1.0f, u), v);
     return u >= 0.0f && v >= 0.0f && tt >= 0.0f && w >= 0.0f;
-}
-__device__ __forceinline__ bool tri_test_exact(const float4& a, const float4& b, const float4& c, f3 org, f3 dir,
-                                               bool cull, float tbest, float& tt, float& u, float& v, float& w) {
-    return tri_hit_exact(a, b, c, org, dir, cull, tt, u, v, w) && tt < tbest;
 }
 
 // the ordering a ray walks: the cube face of its direction (major axis, ties x before y before z;

@@ -64,7 +64,7 @@ struct TraversalCount {
     uint32_t nodes = 0, tris = 0;
 };
 
-// The walk of one ray by one thread.  The divisions of the triangle test (tri_test_exact) follow one
+// The walk of one ray by one thread.  The divisions of the triangle test (tri_hit_exact) follow one
 // another's tests, as few lanes need all three, and the loop ends in one place, so that a warp's lanes
 // meet before the next node (u > 1 leaves w < 0 whatever v is).  AHEAD: both nodes that may come next
 // are loaded before this one is tested (k_trace_photons).
@@ -1816,7 +1816,7 @@ __global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet 
                 const float4 a = __ldg(&tri_isect[(size_t)tri * 3 + 0]);
                 const float4 b = __ldg(&tri_isect[(size_t)tri * 3 + 1]);
                 const float4 c = __ldg(&tri_isect[(size_t)tri * 3 + 2]);
-                // tri_test_exact with the divisions one after the other's test: few lanes get here at a
+                // tri_hit_exact with the divisions one after the other's test: few lanes get here at a
                 // time (3 to 4 of a warp), and often none needs the next one
                 const f3 v0 = mk(a.x, a.y, a.z), e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, c.x);
                 const f3 pv = cross(dir, e1);
