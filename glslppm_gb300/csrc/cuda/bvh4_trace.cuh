@@ -5,7 +5,7 @@
 // node, < 0 ~triangle, INT32_MIN empty); w[2] = lower box bytes x,y,z and upper x; w[3] = upper
 // y,z.  A child box is origin + byte * 2^(exponent-127) per axis, rounded outward when the tree
 // was built; the slab distances are widened by a bound on their rounding, and triangles are
-// tested with the exact path's arithmetic (tri_hit_exact), so the closest hit -- triangle, t and
+// tested with the exact path's arithmetic (device_common.cuh), so the closest hit -- triangle, t and
 // barycentrics -- is the exact traversal's; where two triangles give the same t, the leaf ranks of
 // the exact walk's ordering (DevScene::tri_rank) pick the one it meets first.
 #pragma once
@@ -130,6 +130,10 @@ __device__ __forceinline__ void cswap(float& ta, int32_t& ca, float& tb, int32_t
 
 // closest hit through the 4-wide BVH; PHOTON rays skip emitters, eye rays of the first bounce
 // cull back faces (eyeraytrace.fs:130)
+// The triangle test is the exact walk's, ended at the first coordinate that fails (u > 1 leaves w < 0), a
+// stack entry one 64-bit word, and the loops end without jumps, as in k_trace_photons4.  Us a pass with
+// an eye pass in each, environment scene: 274 -> 265 at 133x234 pixels, 203 -> 199 at 872x96; 1024^2 and
+// larger images the same.
 // rank: the leaf positions of the ordering the exact walk would take for this ray (tri_rank of
 // its cube face) or null; at an equal t the triangle the exact walk meets first wins, as there
 template <bool PHOTON>
@@ -142,12 +146,12 @@ __device__ __forceinline__ Hit4 trace4(const Node4Dev* __restrict__ nodes, const
     h.bu = h.bv = h.bw = 0.0f;
     Ray4 R;
     ray4_setup(R, org.x, org.y, org.z, dir.x, dir.y, dir.z);
-    int32_t stack_node[kStack];
-    float stack_t[kStack];
+    int2 stack[kStack];  // node, entry distance
+    bool found = true;
     int sp = 0;
     int32_t cur = 0;
     uint32_t visits = 0;
-    for (;;) {
+    while (found) {
         if (++visits > 4u * (1u << 20)) {  // bounded: no tree here has this many nodes
             err |= kErrWatchdogTraverse;
             break;
@@ -188,14 +192,26 @@ __device__ __forceinline__ Hit4 trace4(const Node4Dev* __restrict__ nodes, const
             const float4 a = __ldg(&tri_isect[(size_t)tri * 3 + 0]);
             const float4 b = __ldg(&tri_isect[(size_t)tri * 3 + 1]);
             const float4 c = __ldg(&tri_isect[(size_t)tri * 3 + 2]);
-            float tt, u, v, w;
-            if (tri_hit_exact(a, b, c, org, dir, !PHOTON && cull, tt, u, v, w) &&
-                (tt < h.t || (rank && tt == h.t && h.tri >= 0 && __ldg(&rank[tri]) < __ldg(&rank[h.tri])))) {
-                h.t = tt;
-                h.tri = tri;
-                h.bu = v;
-                h.bv = w;
-                h.bw = u;
+            const f3 e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, c.x);
+            const f3 pv = cross(dir, e1);
+            const float det = dot(e0, pv);
+            const f3 tv = sub(org, mk(a.x, a.y, a.z));
+            const f3 qv = cross(tv, e0);
+            const float u = xdiv(dot(tv, pv), det);
+            if (u >= 0.0f && u <= 1.0f && (PHOTON || !cull || det > 1e-10f)) {
+                const float v = xdiv(dot(dir, qv), det);
+                const float w = xsub(xsub(1.0f, u), v);
+                if (v >= 0.0f && w >= 0.0f) {
+                    const float tt = xdiv(dot(e1, qv), det);
+                    if (tt >= 0.0f &&
+                        (tt < h.t || (rank && tt == h.t && h.tri >= 0 && __ldg(&rank[tri]) < __ldg(&rank[h.tri])))) {
+                        h.t = tt;
+                        h.tri = tri;
+                        h.bu = v;
+                        h.bv = w;
+                        h.bw = u;
+                    }
+                }
             }
         }
         // internal children hit before the closest hit so far, sorted near to far: the nearest
@@ -204,34 +220,31 @@ __device__ __forceinline__ Hit4 trace4(const Node4Dev* __restrict__ nodes, const
         const float tcull2 = h.t * kCullMargin;
 #pragma unroll
         for (int k = 0; k < 4; k++)
-            if (!(hit[k] && tnear[k] <= tcull2)) tnear[k] = inf;
+            if (!hit[k]) tnear[k] = inf;
         cswap(tnear[0], ch[0], tnear[1], ch[1]);
         cswap(tnear[2], ch[2], tnear[3], ch[3]);
         cswap(tnear[0], ch[0], tnear[2], ch[2]);
         cswap(tnear[1], ch[1], tnear[3], ch[3]);
         cswap(tnear[1], ch[1], tnear[2], ch[2]);
-        if (tnear[0] < inf) {
-            const int pushes = (tnear[1] < inf) + (tnear[2] < inf) + (tnear[3] < inf);
+        found = tnear[0] <= tcull2;
+        if (found) {
+            const int pushes = (tnear[1] <= tcull2) + (tnear[2] <= tcull2) + (tnear[3] <= tcull2);
             if (sp + pushes > kStack) {
                 err |= kErrWatchdogTraverse;
-                break;
-            }
-            if (tnear[3] < inf) stack_node[sp] = ch[3], stack_t[sp++] = tnear[3];
-            if (tnear[2] < inf) stack_node[sp] = ch[2], stack_t[sp++] = tnear[2];
-            if (tnear[1] < inf) stack_node[sp] = ch[1], stack_t[sp++] = tnear[1];
-            cur = ch[0];
-            continue;
-        }
-        bool found = false;
-        while (sp > 0) {
-            sp--;
-            if (stack_t[sp] <= h.t * kCullMargin) {
-                cur = stack_node[sp];
-                found = true;
-                break;
+                found = false;
+                sp = 0;
+            } else {
+                if (tnear[3] <= tcull2) stack[sp++] = make_int2(ch[3], __float_as_int(tnear[3]));
+                if (tnear[2] <= tcull2) stack[sp++] = make_int2(ch[2], __float_as_int(tnear[2]));
+                if (tnear[1] <= tcull2) stack[sp++] = make_int2(ch[1], __float_as_int(tnear[1]));
+                cur = ch[0];
             }
         }
-        if (!found) break;
+        while (!found && sp > 0) {
+            const int2 e = stack[--sp];
+            cur = e.x;
+            found = __int_as_float(e.y) <= h.t * kCullMargin;
+        }
     }
     return h;
 }

@@ -381,26 +381,14 @@ __device__ __forceinline__ void slab_x(const RayX& R, unsigned long long lo, uns
 __device__ __forceinline__ int32_t node_miss(unsigned long long links) { return (int32_t)(uint32_t)links; }
 __device__ __forceinline__ int32_t node_tri(unsigned long long links) { return (int32_t)(links >> 32); }
 
-// ---- the triangle test of raytrace() (eyeraytrace.fs:200-243, photontrace.fs:196-236) --------
-// Moller-Trumbore on the packed operands (a = v0 | e0.x, b = e0.yz | e1.xy, c.x = e1.z), every
-// operation correctly rounded in the shaders' order, so a triangle's t, u, v and w are the same
-// numbers wherever this is called (plain and mixed traversals alike).  Returns true when the
-// triangle is hit at t >= 0; cull: reject det <= 1e-10 (back faces of a first eye bounce).  The walks of
-// one ray per thread write it out, each division after the one before has passed.
-__device__ __forceinline__ bool tri_hit_exact(const float4& a, const float4& b, const float4& c, f3 org, f3 dir,
-                                              bool cull, float& tt, float& u, float& v, float& w) {
-    const f3 v0 = mk(a.x, a.y, a.z), e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, c.x);
-    const f3 pv = cross(dir, e1);
-    const float det = dot(e0, pv);
-    if (cull && !(det > 1e-10f)) return false;
-    const f3 tv = sub(org, v0);
-    const f3 qv = cross(tv, e0);
-    u = xdiv(dot(tv, pv), det);
-    v = xdiv(dot(dir, qv), det);
-    tt = xdiv(dot(e1, qv), det);
-    w = xsub(xsub(1.0f, u), v);
-    return u >= 0.0f && v >= 0.0f && tt >= 0.0f && w >= 0.0f;
-}
+// The triangle test of raytrace() (eyeraytrace.fs:200-243, photontrace.fs:196-236), which every walk writes
+// out to leave it at its own earliest point: Moller-Trumbore on the packed operands (a = v0 | e0.x,
+// b = e0.yz | e1.xy, c.x = e1.z),
+//     pv = dir x e1, det = e0 . pv, tv = org - v0, qv = tv x e0,
+//     u = tv . pv / det, v = dir . qv / det, t = e1 . qv / det, w = (1 - u) - v,
+// a hit where u, v, w and t are >= 0 (and, culling the back faces of a first eye bounce, det > 1e-10),
+// every operation correctly rounded in this order, so a triangle's t, u, v and w are the same numbers in
+// the plain and the mixed traversals.
 
 // the ordering a ray walks: the cube face of its direction (major axis, ties x before y before z;
 // the negative face when that component is < 0)

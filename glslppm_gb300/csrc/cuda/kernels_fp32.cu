@@ -64,7 +64,7 @@ struct TraversalCount {
     uint32_t nodes = 0, tris = 0;
 };
 
-// The walk of one ray by one thread.  The divisions of the triangle test (tri_hit_exact) follow one
+// The walk of one ray by one thread.  The divisions of the triangle test follow one
 // another's tests, as few lanes need all three, and the loop ends in one place, so that a warp's lanes
 // meet before the next node (u > 1 leaves w < 0 whatever v is).  AHEAD: both nodes that may come next
 // are loaded before this one is tested (k_trace_photons).
@@ -898,7 +898,7 @@ __device__ __forceinline__ bool tile_pixel(const JobDesc& J, uint32_t item, uint
 // mesh 180.8 / 179.3, 189.6 / 190.1, 213.7 / 217.6; 1M triangles 337.2 / 330.8, 343.7 / 338.3, 367.5 / 367.6.
 constexpr uint32_t kEyeAheadItems = 1u << 18;
 // The mixed path's walk has no such chain to shorten, but at 8 blocks it spills 280 bytes of loads: up to
-// kEyeMixedItems it runs with all 93 registers (5 blocks).  Us a pass, 8 / 5 blocks, 1024x512 photons, an
+// kEyeMixedItems it runs with all 91 registers (5 blocks).  Us a pass, 8 / 5 blocks, 1024x512 photons, an
 // eye pass in ten: glass and glossy spheres 228.9 / 227.1 at 256^2 pixels, 244.7 / 239.3 at 512^2,
 // 252.1 / 248.8 at 640x600, but Cornell box 268.4 / 271.1 and 102k-triangle mesh 327.8 / 332.6 at 1536^2;
 // an eye pass in each, 133x234: 287 / 276.
@@ -1816,7 +1816,7 @@ __global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet 
                 const float4 a = __ldg(&tri_isect[(size_t)tri * 3 + 0]);
                 const float4 b = __ldg(&tri_isect[(size_t)tri * 3 + 1]);
                 const float4 c = __ldg(&tri_isect[(size_t)tri * 3 + 2]);
-                // tri_hit_exact with the divisions one after the other's test: few lanes get here at a
+                // the triangle test with the divisions one after the other's test: few lanes get here at a
                 // time (3 to 4 of a warp), and often none needs the next one
                 const f3 v0 = mk(a.x, a.y, a.z), e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, c.x);
                 const f3 pv = cross(dir, e1);

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_photons4(LaunchSet ls, Ra
                 const float4 a = __ldg(&tri_isect[(size_t)code * 3 + 0]);
                 const float4 b = __ldg(&tri_isect[(size_t)code * 3 + 1]);
                 const float4 cc = __ldg(&tri_isect[(size_t)code * 3 + 2]);
-                // tri_hit_exact's arithmetic; u > 1 leaves w < 0 whatever v is
+                // the exact walk's triangle test; u > 1 leaves w < 0 whatever v is
                 const f3 dir = mk(R.dx, R.dy, R.dz);
                 const f3 e0 = mk(a.w, b.x, b.y), e1 = mk(b.z, b.w, cc.x);
                 const f3 pv = cross(dir, e1);
