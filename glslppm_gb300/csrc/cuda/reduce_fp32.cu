@@ -212,31 +212,88 @@ int scratch_address(float4** out) {
     *out = c.ptr;
     return SPPM_OK;
 }
-// The scratch of sppm_reduce_texture: up to kKeptScratch buffers of kScratchTexels per device are kept
-// between calls (an allocation that a synchronization gives back to the system costs the call about
-// 100 us).  A call takes one out of the list and puts it back once its stream has been synchronized,
-// so no two calls share one; they belong to the CUDA context they were made in (after a device reset
-// the list starts anew).
-constexpr size_t kScratchTexels = 256 * 256, kKeptScratch = 4;
+// The scratch of sppm_reduce_texture: up to kKeptScratch buffers per CUDA context are kept between calls
+// (an allocation that a synchronization gives back to the system costs the call 100 us and more), each
+// as large as a call that took it has needed: 256 KiB, 1 MiB from a resolution of 4096, 4 at 8192, 16 at
+// 16384.  A call takes one out of its context's list and puts it back once its stream has been
+// synchronized, so no two calls share one; a call that finds none, kKeptScratch others being under way,
+// allocates its own.  They are the context's (cudaMalloc), so they end with it; a pool's allocations would
+// outlive it.  Context ids are never reused, so the list of a context that is gone is never looked up
+// again; contexts beyond kKeptContexts keep nothing.
+constexpr size_t kLeastScratch = 128 * 128, kKeptScratch = 4, kKeptContexts = 64;
+struct Scratch {
+    float4* ptr;
+    size_t texels;
+};
 struct ScratchList {
     unsigned long long ctx_id;
-    size_t n;
-    float4* free[kKeptScratch];
+    size_t made, n;  // buffers made, and of them free
+    Scratch free[kKeptScratch];
 };
-ScratchList g_scratch_lists[64];  // per device ordinal
+ScratchList g_scratch_lists[kKeptContexts];
+size_t g_scratch_contexts = 0;
 
-// the current device's list (g_scratch_mutex held) and context
-int scratch_list(ScratchList** out, unsigned long long* id) {
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return fail(SPPM_ERR_CUDA, "cudaGetDevice failed: %s", cudaGetErrorString(e));
-    if (dev < 0 || dev >= 64) return fail(SPPM_ERR_ARG, "device ordinal %d out of range", dev);
-    const int st = current_context_id(id);
-    if (st) return st;
-    ScratchList& c = g_scratch_lists[dev];
-    if (c.ctx_id != *id) c = ScratchList{*id, 0, {}};
-    *out = &c;
-    return SPPM_OK;
+// the list of context `id`, null when there is no room for one (g_scratch_mutex held)
+ScratchList* scratch_list(unsigned long long id) {
+    for (size_t i = 0; i < g_scratch_contexts; i++)
+        if (g_scratch_lists[i].ctx_id == id) return &g_scratch_lists[i];
+    if (g_scratch_contexts == kKeptContexts) return nullptr;
+    g_scratch_lists[g_scratch_contexts] = ScratchList{id, 0, 0, {}};
+    return &g_scratch_lists[g_scratch_contexts++];
+}
+
+// a kept buffer for a call on stream s, null when the call has to allocate its own; *id: its context
+Scratch take_scratch(cudaStream_t s, size_t texels, unsigned long long* id) {
+    const Scratch none{nullptr, 0};
+    // (a stream under capture cannot be waited for: the call fails there, as it does without this)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return none;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return none;
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    if (current_context_id(id) != SPPM_OK) return none;
+    if (*id == 0) {  // a thread's first CUDA call: make its device's primary context current
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) {
+            cudaGetLastError();
+            return none;
+        }
+        if (current_context_id(id) != SPPM_OK || *id == 0) return none;
+    }
+    ScratchList* list = scratch_list(*id);
+    if (!list) return none;
+    size_t at = 0;
+    while (at < list->n && list->free[at].texels < texels) at++;
+    if (at < list->n) {
+        const Scratch found = list->free[at];
+        list->free[at] = list->free[--list->n];
+        return found;
+    }
+    if (list->made == kKeptScratch && !list->n) return none;
+    Scratch made{nullptr, texels > kLeastScratch ? texels : kLeastScratch};
+    // another thread's capture does not bear on these calls
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (list->made == kKeptScratch) {  // a larger one in the place of one that is too small
+        cudaFree(list->free[--list->n].ptr);
+        list->made--;
+    }
+    const cudaError_t e = cudaMalloc(&made.ptr, made.texels * sizeof(float4));
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return none;
+    }
+    list->made++;
+    return made;
+}
+
+void put_scratch(unsigned long long id, Scratch scratch) {
+    std::lock_guard<std::mutex> lock(g_scratch_mutex);
+    ScratchList* list = scratch_list(id);
+    list->free[list->n++] = scratch;
 }
 }  // namespace
 
@@ -275,34 +332,21 @@ extern "C" int sppm_reduce_texture(const float* d_texture, uint32_t resolution, 
     if (reinterpret_cast<uintptr_t>(d_texture) & 15) return fail(SPPM_ERR_ARG, "texture must be 16-byte aligned");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t texels = sppm_dev::reduce_scratch_texels(resolution);
-    const bool keep = texels <= kScratchTexels;
-    float4* scratch = nullptr;
-    ScratchList* list = nullptr;
     unsigned long long id = 0;
-    if (keep) {
-        std::lock_guard<std::mutex> lock(g_scratch_mutex);
-        const int st = scratch_list(&list, &id);
-        if (st) return st;
-        if (list->n) scratch = list->free[--list->n];
-    }
+    const Scratch kept = take_scratch(s, texels, &id);
+    float4* scratch = kept.ptr;
     cudaError_t e = cudaSuccess;
-    if (!scratch) e = cudaMallocAsync(&scratch, (keep ? kScratchTexels : texels) * sizeof(float4), s);
+    if (!scratch) e = cudaMallocAsync(&scratch, texels * sizeof(float4), s);
     if (e != cudaSuccess) return fail(SPPM_ERR_OOM, "sppm_reduce_texture: scratch allocation failed: %s", cudaGetErrorString(e));
     sppm_dev::launch_reduce_texture(reinterpret_cast<const float4*>(d_texture), resolution, op, scratch, s);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, scratch, sizeof(float4), cudaMemcpyDeviceToHost, s);
-    if (!keep) cudaFreeAsync(scratch, s);
+    if (!kept.ptr) cudaFreeAsync(scratch, s);
     const cudaError_t e2 = cudaStreamSynchronize(s);
-    if (keep) {
-        std::unique_lock<std::mutex> lock(g_scratch_mutex);
-        if (e == cudaSuccess && e2 == cudaSuccess && id && list->ctx_id == id && list->n < kKeptScratch) {
-            list->free[list->n++] = scratch;
-        } else {
-            lock.unlock();
-            cudaFreeAsync(scratch, s);
-        }
-    }
-    if (e != cudaSuccess || e2 != cudaSuccess)
+    if (kept.ptr && e2 == cudaSuccess) put_scratch(id, kept);  // (else the stream may still work in it)
+    if (e != cudaSuccess || e2 != cudaSuccess) {
+        cudaGetLastError();  // reported here, not by the next call's launch
         return fail(SPPM_ERR_CUDA, "sppm_reduce_texture failed: %s", cudaGetErrorString(e != cudaSuccess ? e : e2));
+    }
     return SPPM_OK;
 }

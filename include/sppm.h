@@ -417,10 +417,11 @@ typedef enum sppm_reduce_op { SPPM_REDUCE_MIN = 0, SPPM_REDUCE_MAX = 1, SPPM_RED
    d_texture holds resolution x resolution float4 texels, row 0 first (16-byte aligned), resolution
    a power of two in [2, 16384].  The texture is folded 2x2 level by level in the order of the
    reference's ping-pong draws, so min, max and sums are bit-identical to it; the 1x1 result is in
-   out[4] (host memory) when the call returns.  Scratch: (resolution/8)^2 float4 (at most 128^2 below
-   2048), allocated stream-ordered on `stream` (cudaStream_t, 0 = default stream); up to resolution
-   2048 the library keeps it for later calls (at most 4 MiB per device), above it is freed before the
-   call returns.  The call synchronizes `stream`. */
+   out[4] (host memory) when the call returns.  Scratch: up to four buffers per CUDA context (one per
+   call under way) are kept for later calls and end with the context, each as large as a call has
+   needed: 256 KiB up to resolution 2048, 1 MiB at 4096, 4 MiB at 8192, 16 MiB at 16384.  A call that
+   finds none free allocates one on `stream` (cudaStream_t, 0 = default stream) and frees it before it
+   returns.  The call synchronizes `stream`. */
 int sppm_reduce_texture(const float* d_texture, uint32_t resolution, uint32_t op, float out[4], void* stream);
 
 /* sppm_reduce_texture for callers that must not allocate device memory -- an engine that reserved
