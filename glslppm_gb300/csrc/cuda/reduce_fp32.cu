@@ -140,12 +140,13 @@ void launch_reduce_texture(const float4* tex, uint32_t resolution, uint32_t op, 
 using sppm::fail;
 
 // ---- variant without device allocation ---------------------------------------------------------
-// Its scratch is this file-scope device array: 512 x 512 float4 = 4 MiB, held by every GPU that
-// loads the library until the process exits.  Host code must not pass `g_reduce_scratch` itself to a
-// kernel (on the host it names a host-side shadow, not device memory): the device address is looked
-// up with cudaGetSymbolAddress once per device and context, with that device current, and cached.
-static __device__ __align__(256) float4 g_reduce_scratch[(SPPM_REDUCE_NOALLOC_MAX_RESOLUTION / 2) *
-                                                         (SPPM_REDUCE_NOALLOC_MAX_RESOLUTION / 2)];
+// Its scratch is this file-scope device array, the first launch's output at any size up to the largest:
+// 128 x 128 float4 = 256 KiB, held by every GPU that loads the library until the process exits.  Host
+// code must not pass `g_reduce_scratch` itself to a kernel (on the host it names a host-side shadow, not
+// device memory): the device address is looked up with cudaGetSymbolAddress once per device and context,
+// with that device current, and cached.
+static __device__ __align__(256) float4 g_reduce_scratch[sppm_dev::kReduceTail * sppm_dev::kReduceTail];
+static_assert(SPPM_REDUCE_NOALLOC_MAX_RESOLUTION <= 16 * sppm_dev::kReduceTail, "the scratch holds the first launch's output");
 
 namespace {
 // The device address of g_reduce_scratch belongs to the CUDA context that loaded the library's
@@ -220,7 +221,7 @@ int scratch_address(float4** out) {
 // allocates its own.  They are the context's (cudaMalloc), so they end with it; a pool's allocations would
 // outlive it.  Context ids are never reused, so the list of a context that is gone is never looked up
 // again; contexts beyond kKeptContexts keep nothing.
-constexpr size_t kLeastScratch = 128 * 128, kKeptScratch = 4, kKeptContexts = 64;
+constexpr size_t kLeastScratch = sppm_dev::kReduceTail * sppm_dev::kReduceTail, kKeptScratch = 4, kKeptContexts = 64;
 struct Scratch {
     float4* ptr;
     size_t texels;

@@ -428,7 +428,7 @@ int sppm_reduce_texture(const float* d_texture, uint32_t resolution, uint32_t op
    the GPU's memory for its own allocator before loading this library, a render loop that forbids
    allocation (and the implicit synchronization cudaMalloc may bring) once it is running.  It has
    no counterpart in the reference, whose ReduceTexture draws into a texture created at start-up.
-   Its scratch is a fixed 4 MiB array in the library's device memory, which every GPU that loads the
+   Its scratch is a fixed 256 KiB array in the library's device memory, which every GPU that loads the
    library keeps until the process exits; resolutions above SPPM_REDUCE_NOALLOC_MAX_RESOLUTION are
    rejected with SPPM_ERR_ARG.  The first call on a device looks up the array's device address
    (cudaGetSymbolAddress, which may load the library's device code) and caches it for the device's
