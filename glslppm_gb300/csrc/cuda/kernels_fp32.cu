@@ -1696,7 +1696,8 @@ __global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet 
     const unsigned lane = threadIdx.x & 31;
     const uint32_t kNeed = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu;
     // fewer rays than lanes: spread over all warps (spread_lanes)
-    uint32_t idx = lane < spread_lanes(total) ? kNeed : kDone;
+    const bool takes_rays = lane < spread_lanes(total);
+    uint32_t idx = takes_rays ? kNeed : kDone;
     const NodeX* nodes = nullptr;
     const float4* tri_isect = nullptr;
     int32_t nn = 0;
@@ -1776,7 +1777,8 @@ __global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet 
         // dependent node loads becomes windows of 32 loads in flight
         if (q.tail_lanes) {
             const unsigned act = __ballot_sync(0xFFFFFFFFu, idx < kDone);
-            const unsigned drained = __ballot_sync(0xFFFFFFFFu, idx == kDone);
+            // (a lane that takes rays has found none left)
+            const unsigned drained = __ballot_sync(0xFFFFFFFFu, idx == kDone && takes_rays);
             if (drained && act && (uint32_t)__popc(act) <= q.tail_lanes) {
                 if (idx < kDone) {
                     const int32_t mat = h.tri >= 0 ? __float_as_int(__ldg(&tri_isect[(size_t)h.tri * 3 + 2]).y) : -1;

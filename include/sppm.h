@@ -352,8 +352,8 @@ typedef struct sppm_tuning {
                                      shapes are set the library chooses (and reports 0): bins for
                                      the plain path's single job with 3/4 * 2^20 photon slots or
                                      more, else queue order (same results)                      */
-    uint32_t trace_tail_lanes;    /* exact traversal: once the ray queue is drained, a warp with
-                                     at most this many walking lanes hands those walks to a tail
+    uint32_t trace_tail_lanes;    /* exact traversal: once a lane has found the ray queue drained, its
+                                     warp, if at most this many lanes walk, hands those walks to a tail
                                      kernel that finishes each with all 32 lanes of a warp (the
                                      warp-cooperative walk; same results) (0 = off, up to 32)   */
     uint32_t wide_bvh;            /* plain FP32 path: 1 traces eye and photon rays through the
