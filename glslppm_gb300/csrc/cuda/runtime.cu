@@ -1089,8 +1089,14 @@ void Runner::timed(int stage, bool start, cudaStream_t s) {
 constexpr uint32_t kBinnedSlots = 768 * 1024;
 constexpr uint32_t kMixedQueueRefill = 4;
 bool Runner::rays_in_queue_order() const {
+    if (flags & SPPM_FLAG_UNBINNED_RAYS) return true;
     if (shapes_set) return tune.unbinned_rays != 0;
     return precision == SPPM_PRECISION_MIXED || active.size() > 1 || pho.total < kBinnedSlots;
+}
+uint32_t Runner::refill_steps(bool wide, bool queue_order) const {
+    if (tune.trace_refill_steps) return tune.trace_refill_steps;
+    if (precision == SPPM_PRECISION_MIXED) return queue_order ? kMixedQueueRefill : 8u;
+    return wide ? 8u : 32u;
 }
 
 // Launches of up to this many photon slots take the walk that loads a step ahead: there the longest walk's
@@ -1111,10 +1117,13 @@ int Runner::enqueue_frame(uint32_t phase) {
     // the queue as the launches see it: the tuned refill interval, and no bins when the rays are
     // traced in queue order
     RayQueue q = queue;
-    q.refill_steps = tune.trace_refill_steps;
     q.tail_lanes = tune.trace_tail_lanes;
+    const bool mixed = precision == SPPM_PRECISION_MIXED;
+    // the plain path through the 4-wide BVH (the same hits): not for the traversal-counting pass,
+    // which measures the binary walk
+    const bool wide = mixed || (tune.wide_bvh && wide_ok && !count_traversal);
     const bool queue_order = rays_in_queue_order();
-    if (!q.refill_steps && queue_order && precision == SPPM_PRECISION_MIXED) q.refill_steps = kMixedQueueRefill;
+    q.refill_steps = refill_steps(wide, queue_order);
     if (queue_order) {
         q.key = nullptr;
         q.perm = nullptr;
@@ -1128,10 +1137,6 @@ int Runner::enqueue_frame(uint32_t phase) {
     // the eye pass and the grid it sets run beside the photon generation and traversal (which do
     // not read them); the photon store (hash insertion) waits for the grid
     const bool eye = phase_has_eye(phase);
-    const bool mixed = precision == SPPM_PRECISION_MIXED;
-    // the plain path through the 4-wide BVH (the same hits): not for the traversal-counting pass,
-    // which measures the binary walk
-    const bool wide = mixed || (tune.wide_bvh && wide_ok && !count_traversal);
     const uint32_t wide_blocks = std::min(trace_blocks, sms * trace_fit4);
     if (eye) {
         SPPM_CK(cudaEventRecord(fork_ev, stream));
@@ -1257,6 +1262,7 @@ int Runner::run(uint32_t n) {
     int st;
     if (dirty && (st = rebuild())) return st;
     if (active.empty()) return SPPM_OK;
+    ran = true;
     // the kernel variants with texture lookups when some job's scene has texture coordinates
     textured = false;
     for (const Job* j : active) textured = textured || j->desc.scene.tri_tex != nullptr;
@@ -1342,6 +1348,11 @@ int Runner::set_tuning(const sppm_tuning* t) {
     if (t->wide_bvh > 1) return fail(SPPM_ERR_ARG, "wide_bvh is 0 or 1");
     if (t->grid_cell_split > 8 || (t->grid_cell_split & (t->grid_cell_split - 1)))
         return fail(SPPM_ERR_ARG, "grid_cell_split is 0 (default), 1, 2, 4 or 8");
+    if (!shapes_set) {  // what get_tuning reports, handed back, changes nothing
+        sppm_tuning now;
+        get_tuning(&now);
+        if (memcmp(t, &now, sizeof(now)) == 0) return SPPM_OK;
+    }
     SPPM_CK(cudaSetDevice(device));
     SPPM_CK(cudaStreamSynchronize(stream));
     tune = *t;
@@ -1352,14 +1363,19 @@ int Runner::set_tuning(const sppm_tuning* t) {
 }
 
 void Runner::get_tuning(sppm_tuning* t) const {
+    // (the library chooses an order for the jobs of a run: none before the first)
+    shapes_with(t, rays_in_queue_order() && (shapes_set || ran || (flags & SPPM_FLAG_UNBINNED_RAYS)));
+}
+
+void Runner::shapes_with(sppm_tuning* t, bool queue_order) const {
     *t = tune;
     if (!t->trace_blocks_per_sm) t->trace_blocks_per_sm = trace_fit;
-    if (!t->trace_refill_steps) t->trace_refill_steps = precision == SPPM_PRECISION_MIXED ? 8u : 32u;
+    t->trace_refill_steps = refill_steps(tune.wide_bvh && wide_ok, queue_order);
+    t->unbinned_rays = queue_order;
     if (!t->eye_block) t->eye_block = 128;
     if (!t->store_block) t->store_block = 128;
     if (!t->gather_block) t->gather_block = 256;
     if (!t->grid_cell_split) t->grid_cell_split = kDefaultGridCellSplit;
-    if (flags & SPPM_FLAG_UNBINNED_RAYS) t->unbinned_rays = 1;  // created without ray bins
 }
 
 int Runner::autotune(uint32_t cycles, sppm_tuning* best, float* ms_per_pass) {
@@ -1371,7 +1387,7 @@ int Runner::autotune(uint32_t cycles, sppm_tuning* best, float* ms_per_pass) {
     // a window of whole eye-pass cycles holds every phase equally often, wherever it starts
     const uint32_t L = eye_interval, window = cycles * L;
     sppm_tuning cur;
-    get_tuning(&cur);
+    shapes_with(&cur, rays_in_queue_order());
     auto measure = [&](const sppm_tuning& t, float* ms) -> int {
         int e = set_tuning(&t);
         if (e) return e;

@@ -245,7 +245,10 @@ struct Runner {
     uint32_t sms = 0, trace_fit = 0;  // SMs; traversal blocks of 128 threads that fit on one SM
     sppm_tuning tune{};               // launch shapes (zero fields: the defaults)
     bool shapes_set = false;          // set_tuning was called: tune.unbinned_rays is the order of the rays
+    bool ran = false;                 // a frame has been launched
     bool rays_in_queue_order() const; // the next frame's photon rays are not binned
+    uint32_t refill_steps(bool wide, bool queue_order) const;  // the traversal's refill interval
+    void shapes_with(sppm_tuning* t, bool queue_order) const;  // the shapes, defaults filled in, with this order
     bool dirty = true;
     // stage timing
     uint32_t timing_mask = 0;  // bit k: time stage k

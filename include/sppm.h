@@ -348,10 +348,10 @@ typedef struct sppm_tuning {
     uint32_t store_block;         /* of the photon store + hash insertion (0 = 128; 32..128)    */
     uint32_t gather_block;        /* of the gather + progressive update (0 = 256; 32..256; of the
                                      counting-sort grid at most 128)                            */
-    uint32_t unbinned_rays;       /* 1: photon rays traced in queue order instead of binned.  Until
-                                     shapes are set the library chooses (and reports 0): bins for
+    uint32_t unbinned_rays;       /* 1: photon rays traced in queue order, 0: binned (same results).
+                                     Until shapes are set the library chooses at each run: bins for
                                      the plain path's single job with 3/4 * 2^20 photon slots or
-                                     more, else queue order (same results)                      */
+                                     more, else queue order.  Setting shapes sets the order too     */
     uint32_t trace_tail_lanes;    /* exact traversal: once a lane has found the ray queue drained, its
                                      warp, if at most this many lanes walk, hands those walks to a tail
                                      kernel that finishes each with all 32 lanes of a warp (the
@@ -380,7 +380,10 @@ typedef struct sppm_tuning {
 } sppm_tuning;
 /* Block sizes are multiples of 32.  The frame graphs are captured again with the new shapes. */
 int sppm_set_tuning(sppm_ctx* ctx, const sppm_tuning* tuning);
-/* The shapes in effect (defaults filled in). */
+/* The shapes in effect (defaults filled in): from the first run on with the order of the rays that the
+   library chose, where none was set; before it with unbinned_rays 0.  Setting what is reported changes
+   nothing, so to change one shape and keep the order, change it in the report of a context that has
+   run. */
 int sppm_get_tuning(sppm_ctx* ctx, sppm_tuning* tuning);
 /* Runs the context's next passes under candidate shapes and leaves the fastest in effect:
    a grid over ray order x refill interval, then coordinate descent over the other fields (a
