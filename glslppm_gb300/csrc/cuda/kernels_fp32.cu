@@ -1694,10 +1694,10 @@ __global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet 
     const uint32_t total = q.counters[0];
     const int refill = q.refill_steps ? (int)q.refill_steps : 32;
     const unsigned lane = threadIdx.x & 31;
-    const uint32_t kNeed = 0xFFFFFFFFu, kDone = 0xFFFFFFFEu;
-    // fewer rays than lanes: spread over all warps (spread_lanes)
-    const bool takes_rays = lane < spread_lanes(total);
-    uint32_t idx = takes_rays ? kNeed : kDone;
+    // a lane's ray, or: it needs one, it has found none left, it takes none (with fewer rays than lanes
+    // they are spread over all warps, spread_lanes)
+    const uint32_t kNeed = 0xFFFFFFFDu, kDone = 0xFFFFFFFEu, kIdle = 0xFFFFFFFFu;
+    uint32_t idx = lane < spread_lanes(total) ? kNeed : kIdle;
     const NodeX* nodes = nullptr;
     const float4* tri_isect = nullptr;
     int32_t nn = 0;
@@ -1770,17 +1770,16 @@ __global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet 
                 }
             }
         }
-        if (__all_sync(0xFFFFFFFFu, idx == kDone)) break;
+        if (__all_sync(0xFFFFFFFFu, idx >= kDone)) break;
         // the tail: once the queue is drained, a warp left with a few long walks hands them to
         // k_trace_photons_tail, which finishes each with all 32 lanes of a warp, resumed where the
         // lane stands (coop_trace_exact_from, the same result bit for bit): a walk's chain of
         // dependent node loads becomes windows of 32 loads in flight
         if (q.tail_lanes) {
-            const unsigned act = __ballot_sync(0xFFFFFFFFu, idx < kDone);
-            // (a lane that takes rays has found none left)
-            const unsigned drained = __ballot_sync(0xFFFFFFFFu, idx == kDone && takes_rays);
+            const unsigned act = __ballot_sync(0xFFFFFFFFu, idx < kNeed);
+            const unsigned drained = __ballot_sync(0xFFFFFFFFu, idx == kDone);
             if (drained && act && (uint32_t)__popc(act) <= q.tail_lanes) {
-                if (idx < kDone) {
+                if (idx < kNeed) {
                     const int32_t mat = h.tri >= 0 ? __float_as_int(__ldg(&tri_isect[(size_t)h.tri * 3 + 2]).y) : -1;
                     q.hit[idx] = make_float4(__int_as_float(h.tri), h.bu, h.bv, h.bw);
                     q.tail_state[idx] = make_float4(h.t, __int_as_float(mat), __int_as_float(node),
@@ -1791,7 +1790,7 @@ __global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet 
                 continue;  // every walk of the warp is handed over; the next iteration leaves the loop
             }
         }
-        if (idx >= kDone) continue;
+        if (idx >= kNeed) continue;
         bool finished = false;
         int it = 0;
         unsigned long long lo, hi, near_far, links;
