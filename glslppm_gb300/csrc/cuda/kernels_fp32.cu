@@ -890,8 +890,11 @@ __device__ __forceinline__ bool tile_pixel(const JobDesc& J, uint32_t item, uint
 // its rays spread less than a row of 32 pixels does, so they share more nodes and end closer together.
 // Us a pass of ten with one eye frame, rows -> tiles: a 1024^2 frame of a 1M-triangle mesh 1057 -> 1049,
 // sixteen 512^2 frames 1043 -> 1029, the Cornell box at 1024^2 302 -> 301; and 8 resident blocks
-// (64 registers, 12 bytes spilled) 1049 -> 1044, 1029 -> 1025, 301 -> 301.  The textured path needs more
-// registers than that.
+// (64 registers, 12 bytes spilled) 1049 -> 1044, 1029 -> 1025, 301 -> 301.  The textured path gets 6 (80
+// registers): us a pass of the textured box with an eye pass in each and 1024^2 photons, 5 / 6 / 8 blocks,
+// plain 505 / 489 / 475 at 1024^2 pixels and 697 / 666 / 636 at 1536^2, mixed 514 / 502 / 500 and
+// 715 / 691 / 684; with 512^2 photons 179.4 / 178.5 / 184.6 and 181.5 / 180.0 / 181.2 at 512^2, with 256^2
+// 126.0 / 126.2 / 127.5 and 102.5 / 102.8 / 103.9 at 256^2.
 // AHEAD (launches of up to kEyeAheadItems, untextured): with few warps the paths' chains decide.  Us a pass
 // without / with it, 512^2 photons: glass and glossy spheres 166.8 / 157.6 at 256^2 pixels, 173.2 / 167.4
 // at 512^2, 196.9 / 194.3 at 1024x768; Cornell box 121.9 / 121.4, 125.7 / 126.0, 148.3 / 149.7; 102k-triangle
@@ -904,7 +907,7 @@ constexpr uint32_t kEyeAheadItems = 1u << 18;
 // an eye pass in each, 133x234: 287 / 276.
 constexpr uint32_t kEyeMixedItems = 1u << 19;
 template <bool MIXED, bool TEX, bool AHEAD = false>
-__global__ void __launch_bounds__(128, TEX ? 5 : AHEAD ? (MIXED ? 5 : 6) : 8)
+__global__ void __launch_bounds__(128, TEX ? 6 : AHEAD ? (MIXED ? 5 : 6) : 8)
     k_eye(LaunchSet ls, uint32_t* deferred_n, uint32_t* deferred, uint32_t deferred_cap) {
     // the block's segment count for the job of its first item: one global add per block, made by the
     // last of its threads to get there (no barrier: the others' registers are free when their paths
@@ -1410,8 +1413,12 @@ __global__ void __launch_bounds__(128) k_photon(LaunchSet ls) {
 // glossy spheres with 517x389 photons 163.9 -> 159.4, a 1M-triangle mesh with 2^21 photons 1039 -> 1036.
 // Blocks of 64 threads (twice the adds to the queue's counter): 297.5, 1024, 162.7, 1059 where
 // these read 293.2, 1008, 160.3, 1046; of 512: 306, 1035, 159.6, 1043.
+// Textured, 6 blocks (80 registers): us a pass of the textured box, an eye pass in each, 5 / 6 / 8 blocks,
+// 504 / 489 / 480 with 1024^2 photons and pixels, 179.0 / 177.5 / 177.0 with 512^2 (mixed 515 / 500 / 492 and
+// 181.8 / 177.6 / 177.9), 125.8 / 126.2 / 126.4 with 256^2; 8 blocks spill 156 bytes and take the small launches'
+// generation 4 to 9 % longer (20.0 -> 21.5 us with 128^2, 24.9 -> 27.3 with 256^2).
 template <bool TEX>
-__global__ void __launch_bounds__(128, TEX ? 5 : 10) k_photon_gen(LaunchSet ls, RayQueue q) {
+__global__ void __launch_bounds__(128, TEX ? 6 : 10) k_photon_gen(LaunchSet ls, RayQueue q) {
     // the slots and their previous hits in processing order
     __shared__ uint32_t order[128];
     __shared__ int2 rec_hit[128];
