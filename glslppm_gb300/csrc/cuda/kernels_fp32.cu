@@ -627,7 +627,7 @@ __device__ __forceinline__ float xorshift_frand(uint32_t* s) {
     return xmul(__uint2float_rn(s[3]), 1.0f / 4294967295.0f);
 }
 
-// (four hash slots and four bins a thread: one search for the job and two wide stores)
+// a job's state at the start of a frame
 __device__ __forceinline__ void begin_job(const JobDesc& J) {
     JobState* st = J.state;
     const uint32_t f = st->frames_started;
@@ -648,6 +648,7 @@ __device__ __forceinline__ void begin_job(const JobDesc& J) {
         }
     }
 }
+// (four hash slots and four bins a thread: one search for the job and two wide stores)
 __global__ void k_frame_begin(LaunchSet ls, RayQueue q) {
     const uint32_t t = grid_tid();
     if (t == 0 && q.counters) {
@@ -886,28 +887,33 @@ __device__ __forceinline__ bool tile_pixel(const JobDesc& J, uint32_t item, uint
 // (their whole path is rerun there with block-wide walks); the mixed path's slab tests do not
 // degenerate.
 //
-// Bound by the divergence of a warp's paths and by the node loads' latency.  A warp takes an 8x4 tile:
-// its rays spread less than a row of 32 pixels does, so they share more nodes and end closer together.
-// Us a pass of ten with one eye frame, rows -> tiles: a 1024^2 frame of a 1M-triangle mesh 1057 -> 1049,
-// sixteen 512^2 frames 1043 -> 1029, the Cornell box at 1024^2 302 -> 301; and 8 resident blocks
-// (64 registers, 12 bytes spilled) 1049 -> 1044, 1029 -> 1025, 301 -> 301.  The textured path gets 6 (80
-// registers): us a pass of the textured box with an eye pass in each and 1024^2 photons, 5 / 6 / 8 blocks,
-// plain 505 / 489 / 475 at 1024^2 pixels and 697 / 666 / 636 at 1536^2, mixed 514 / 502 / 500 and
+// Bound by the divergence of a warp's paths and by the node loads' latency.  A warp takes an 8x4 tile: its
+// rays spread less than a row of 32 pixels does, so they share more nodes and end closer together.  Us a
+// pass of ten with one eye frame, rows -> tiles: a 1024^2 frame of a 1M-triangle mesh 1057 -> 1049, sixteen
+// 512^2 frames 1043 -> 1029, the Cornell box at 1024^2 302 -> 301; and 8 resident blocks (64 registers;
+// spills of 44 bytes stored, 28 loaded) 1049 -> 1044, 1029 -> 1025, 301 -> 301.  The textured path gets 6
+// (80 registers): us a pass of the textured box with an eye pass in each and 1024^2 photons, 5 / 6 / 8
+// blocks, plain 505 / 489 / 475 at 1024^2 pixels and 697 / 666 / 636 at 1536^2, mixed 514 / 502 / 500 and
 // 715 / 691 / 684; with 512^2 photons 179.4 / 178.5 / 184.6 and 181.5 / 180.0 / 181.2 at 512^2, with 256^2
 // 126.0 / 126.2 / 127.5 and 102.5 / 102.8 / 103.9 at 256^2.
-// AHEAD (launches of up to kEyeAheadItems, untextured): with few warps the paths' chains decide.  Us a pass
-// without / with it, 512^2 photons: glass and glossy spheres 166.8 / 157.6 at 256^2 pixels, 173.2 / 167.4
-// at 512^2, 196.9 / 194.3 at 1024x768; Cornell box 121.9 / 121.4, 125.7 / 126.0, 148.3 / 149.7; 102k-triangle
-// mesh 180.8 / 179.3, 189.6 / 190.1, 213.7 / 217.6; 1M triangles 337.2 / 330.8, 343.7 / 338.3, 367.5 / 367.6.
+// FEW (untextured launches of few items): the exact path walks a step ahead, the mixed one has more
+// registers.
+//
+// Up to kEyeAheadItems the exact path's walk loads a step ahead: with few warps the paths' chains decide.
+// Us a pass without / with it, an eye pass in each, 1024x512 photons: glass and glossy spheres 433 / 366 at
+// 256^2 pixels, 465 / 407 at 512^2, 514 / 479 at 768^2, 604 / 597 at 1024^2, 901 / 937 at 1536^2; Cornell
+// box 172 / 174, 192 / 198, 232 / 243, 289 / 307, 422 / 463; 102k-triangle mesh 282 / 266, 308 / 321, 369 / 400,
+// 449 / 500, 654 / 754.  Up to 2^18 the long paths gain more than the short ones lose (with an eye pass in
+// ten: glass 232 / 225 at 256^2, 243 / 237 at 512^2, box 164 / 164, 169 / 170, mesh 244 / 245, 252 / 253).
 constexpr uint32_t kEyeAheadItems = 1u << 18;
-// The mixed path's walk has no such chain to shorten, but at 8 blocks it spills 280 bytes of loads: up to
-// kEyeMixedItems it runs with all 91 registers (5 blocks).  Us a pass, 8 / 5 blocks, 1024x512 photons, an
-// eye pass in ten: glass and glossy spheres 228.9 / 227.1 at 256^2 pixels, 244.7 / 239.3 at 512^2,
-// 252.1 / 248.8 at 640x600, but Cornell box 268.4 / 271.1 and 102k-triangle mesh 327.8 / 332.6 at 1536^2;
-// an eye pass in each, 133x234: 287 / 276.
+// The mixed path's walk has no such chain to shorten, but at 8 blocks it spills (112 bytes stored, 280
+// loaded): up to kEyeMixedItems it runs with all 91 registers (5 blocks).  Us a pass, 8 / 5 blocks, as above:
+// glass and glossy spheres 368 / 356 at 256^2, 443 / 406 at 512^2, 474 / 436 at 640x600, 526 / 492 at 768^2,
+// 661 / 631 at 1024^2, 1022 / 1041 at 1536^2; Cornell box 175 / 173, 202 / 201, 216 / 217, 242 / 247, 298 / 311,
+// 459 / 483; 102k-triangle mesh 262 / 259, 315 / 315, 341 / 344, 389 / 394, 483 / 499, 738 / 780.
 constexpr uint32_t kEyeMixedItems = 1u << 19;
-template <bool MIXED, bool TEX, bool AHEAD = false>
-__global__ void __launch_bounds__(128, TEX ? 6 : AHEAD ? (MIXED ? 5 : 6) : 8)
+template <bool MIXED, bool TEX, bool FEW = false>
+__global__ void __launch_bounds__(128, TEX ? 6 : FEW ? (MIXED ? 5 : 6) : 8)
     k_eye(LaunchSet ls, uint32_t* deferred_n, uint32_t* deferred, uint32_t deferred_cap) {
     // the block's segment count for the job of its first item: one global add per block, made by the
     // last of its threads to get there (no barrier: the others' registers are free when their paths
@@ -935,7 +941,7 @@ __global__ void __launch_bounds__(128, TEX ? 6 : AHEAD ? (MIXED ? 5 : 6) : 8)
                 return false;
             }
         }
-        h = trace_exact<false, false, AHEAD>(J.scene, org, dir, cull, err);
+        h = trace_exact<false, false, FEW>(J.scene, org, dir, cull, err);
         return true;
     }, o);
     if (done) eye_write(J, st, p, o);
@@ -1408,15 +1414,15 @@ __global__ void __launch_bounds__(128) k_photon(LaunchSet ls) {
 // works on it (within the block's lines; an emission reads none of it but the generator).
 //
 // Bound by the instructions of the two paths and the latency of these loads: 10 blocks per SM (48
-// registers).  Us a pass against the whole record staged through shared memory at 9 blocks (56
-// registers) -> this: the Cornell box at 1024^2 297.1 -> 290.8, sixteen jobs 1013 -> 1002, glass and
-// glossy spheres with 517x389 photons 163.9 -> 159.4, a 1M-triangle mesh with 2^21 photons 1039 -> 1036.
-// Blocks of 64 threads (twice the adds to the queue's counter): 297.5, 1024, 162.7, 1059 where
-// these read 293.2, 1008, 160.3, 1046; of 512: 306, 1035, 159.6, 1043.
+// registers; spills of 20 bytes stored, 28 loaded).  Us a pass against the whole record staged through
+// shared memory at 9 blocks (56 registers) -> this: the Cornell box at 1024^2 297.1 -> 290.8, sixteen jobs
+// 1013 -> 1002, glass and glossy spheres with 517x389 photons 163.9 -> 159.4, a 1M-triangle mesh with 2^21
+// photons 1039 -> 1036.  Blocks of 64 threads (twice the adds to the queue's counter): 297.5, 1024, 162.7,
+// 1059 where these read 293.2, 1008, 160.3, 1046; of 512: 306, 1035, 159.6, 1043.
 // Textured, 6 blocks (80 registers): us a pass of the textured box, an eye pass in each, 5 / 6 / 8 blocks,
 // 504 / 489 / 480 with 1024^2 photons and pixels, 179.0 / 177.5 / 177.0 with 512^2 (mixed 515 / 500 / 492 and
-// 181.8 / 177.6 / 177.9), 125.8 / 126.2 / 126.4 with 256^2; 8 blocks spill 156 bytes and take the small launches'
-// generation 4 to 9 % longer (20.0 -> 21.5 us with 128^2, 24.9 -> 27.3 with 256^2).
+// 181.8 / 177.6 / 177.9), 125.8 / 126.2 / 126.4 with 256^2; 8 blocks spill 156 bytes and take the small
+// launches' generation 4 to 9 % longer (20.0 -> 21.5 us with 128^2, 24.9 -> 27.3 with 256^2).
 template <bool TEX>
 __global__ void __launch_bounds__(128, TEX ? 6 : 10) k_photon_gen(LaunchSet ls, RayQueue q) {
     // the slots and their previous hits in processing order
@@ -1695,7 +1701,7 @@ __global__ void __launch_bounds__(256) k_ray_bins_scatter(RayQueue q) {
 // 2^16 63 instead of 74.
 // AHEAD (launches of up to kTraceAheadSlots): a step loads both nodes that the next one may need before
 // it tests its own box, so the chain of a walk holds the loads alone and not the test between them; twice
-// the loads and 80 registers (6 blocks per SM) that larger launches have no room for.
+// the loads and 75 registers (6 blocks per SM) that larger launches have no room for.
 template <bool COUNT, bool AHEAD>
 __global__ void __launch_bounds__(128, AHEAD ? 6 : 9) k_trace_photons(LaunchSet ls, RayQueue q) {
     const uint32_t total = q.counters[0];
@@ -1964,10 +1970,11 @@ __global__ void __launch_bounds__(128) k_photon_store(LaunchSet ls, RayQueue q, 
 // loads -- pixel state, the eight cells' winners, their photons -- at 32 warps per SM (64 registers);
 // the bounds of the in-cell test are nine planes per pixel, loaded once, not six per cell: 57.8 -> 52.1
 // us on the Cornell box (1024^2), 189 -> 171 over 16 jobs.
-// BLOCKS per SM: 5 (48 registers, 52 bytes spilled) where a launch has waves of blocks to fill them.  Us a
-// pass with 1024x512 photons, 4 / 5 blocks: Cornell box 168.1 / 171.4 at 512^2 pixels, 186.9 / 189.2 at
-// 768^2, 210.1 / 209.2 at 1024^2, 216.2 / 214.7 at 1280x1024, 343.8 / 332.9 at 2048^2; 102k-triangle mesh
-// 256.3 / 254.8, 269.0 / 268.9, 288.5 / 285.7, 297.5 / 295.2, 407.0 / 397.5; sixteen jobs 978 / 968.
+// BLOCKS per SM: 5 (48 registers; spills of 52 bytes stored, 72 loaded) where a launch has waves of blocks
+// to fill them.  Us a pass with 1024x512 photons, 4 / 5 blocks: Cornell box 168.1 / 171.4 at 512^2 pixels,
+// 186.9 / 189.2 at 768^2, 210.1 / 209.2 at 1024^2, 216.2 / 214.7 at 1280x1024, 343.8 / 332.9 at 2048^2;
+// 102k-triangle mesh 256.3 / 254.8, 269.0 / 268.9, 288.5 / 285.7, 297.5 / 295.2, 407.0 / 397.5; sixteen
+// jobs 978 / 968.
 constexpr uint32_t kGatherWideItems = 1u << 20;
 template <int BLOCKS>
 __global__ void __launch_bounds__(256, BLOCKS) k_gather(LaunchSet ls) {

@@ -389,10 +389,12 @@ __device__ __forceinline__ void grid_accumulate(const PhotonGrid& grid, uint32_t
 // 181 us with every pixel decoding what it takes, in blocks of 256 threads; 157 decoded once; 150 with
 // 5 such blocks per SM for 4; 142 in blocks of 128, whose tiles wait for fewer others (64: 142, 32: 148).
 constexpr uint32_t kCoopMaxCells = 128;
-// From this many pixels the blocks are bounded to 48 registers (10 per SM; 64 bytes spilled).  Us a pass with
-// 1024x512 photons, 8 / 10 blocks: Cornell box 235.1 / 240.0 at 640x600 pixels, 250.3 / 252.3 at 768^2,
-// 273.9 / 272.8 at 1024^2, 347 / 337 at 1536^2; glass and glossy spheres 317 / 319, 340.5 / 339.6, 393 / 386,
-// 545 / 529; 102k-triangle mesh 337 / 344, 349 / 354, 381.0 / 382.8, 448 / 446.
+// From this many pixels the blocks are bounded to 48 registers (10 per SM; spills of 52 bytes stored, 48
+// loaded).  Us a pass with 1024x512 photons, 8 / 10 blocks: Cornell box 235.5 / 235.3 at 640x600 pixels, 250.9 /
+// 252.1 at 768^2, 252.4 / 253.5 at 1024x768, 269.0 / 268.5 at 1024^2, 274 / 273 at 1152x1024, 293 / 287 at
+// 1200^2, 343 / 334 at 1536^2; glass and glossy spheres 310 / 314, 334 / 333, 342 / 339, 382 / 377, 397 / 386,
+// 424 / 419, 528 / 514; 102k-triangle mesh 327 / 332, 341 / 347, 346 / 353, 368 / 371, 369 / 372, 389 / 392,
+// 432 / 432: at 2^20 the box and the spheres gain what the mesh loses.
 constexpr uint32_t kGridWideItems = 1u << 20;
 constexpr uint32_t kGridGatherBlock = 128;  // threads (at most) of the grid gather's blocks
 

@@ -1081,11 +1081,12 @@ void Runner::timed(int stage, bool start, cudaStream_t s) {
 
 // The order of the rays until the shapes are set.  Binning costs three more kernels and the ranks in the
 // generation (16 to 23 us and a few per cent of it); what it saves grows with the rays of one scene.
-// Measured (us a pass, binned / queue order, 512^2 images): Cornell box 122 / 108 at 2^17 slots, 192 / 187
-// at 2^19, 277 / 295 at 2^20; 102k-triangle mesh 423 / 394 at 2^19 and 1M triangles 1071 / 1132 at 2^21;
-// 16 jobs of 12k to 100k triangles 1114 / 1058.  The 4-wide walk, which takes the nearest child first, gains
-// nothing from bins: Cornell box 352 / 346 (2^20), 1M-triangle mesh 1242 / 937 (2^21), refilled every
-// 4 steps (8 steps: 964).
+// Measured (us a pass, binned / queue order, 512^2 images): Cornell box 122 / 108 at 2^17 slots, 169 / 169
+// at 2^19, 216 / 220 at 3/4 * 2^20, 246 / 266 at 2^20, 421 / 454 at 2^21; glass and glossy spheres 226 / 235,
+// 299 / 313, 372 / 393, 675 / 705 from 2^19 on; 1M triangles 1071 / 1132 at 2^21; but a 102k-triangle mesh
+// 275 / 253, 332 / 308, 402 / 366, 653 / 600 and 16 jobs of 12k to 100k triangles 1114 / 1058.  The 4-wide
+// walk, which takes the nearest child first, gains nothing from bins: Cornell box 352 / 346 (2^20),
+// 1M-triangle mesh 1242 / 937 (2^21), refilled every 4 steps (8 steps: 964).
 constexpr uint32_t kBinnedSlots = 768 * 1024;
 constexpr uint32_t kMixedQueueRefill = 4;
 bool Runner::rays_in_queue_order() const {
