@@ -2112,16 +2112,17 @@ __global__ void k_resolve(LaunchSet ls, uint32_t display) {
 // ----------------------------------------------------------------------------------------------
 // stage-level hash build on caller arrays (sppm_hash_build)
 // ----------------------------------------------------------------------------------------------
-// (four slots a thread where the arrays allow it)
+// (four slots a thread where the arrays allow it; a table may have up to 2^32 - 1)
 __global__ void k_hash_clear(uint32_t* winner, uint32_t* count, uint32_t n) {
     const uint32_t g = grid_tid() * 4u;
-    if (g + 4u <= n && ((reinterpret_cast<uintptr_t>(winner) | reinterpret_cast<uintptr_t>(count)) & 15) == 0) {
+    if (g >= n) return;
+    if (n - g >= 4u && ((reinterpret_cast<uintptr_t>(winner) | reinterpret_cast<uintptr_t>(count)) & 15) == 0) {
         *reinterpret_cast<uint4*>(winner + g) = make_uint4(kEmptySlot, kEmptySlot, kEmptySlot, kEmptySlot);
         *reinterpret_cast<uint4*>(count + g) = make_uint4(0u, 0u, 0u, 0u);
     } else {
-        for (uint32_t i = g; i < n && i < g + 4u; i++) {
-            winner[i] = kEmptySlot;
-            count[i] = 0;
+        for (uint32_t i = 0; i < 4u && i < n - g; i++) {
+            winner[g + i] = kEmptySlot;
+            count[g + i] = 0;
         }
     }
 }
@@ -2369,7 +2370,7 @@ void launch_resolve_fp32(const LaunchSet& ls, uint32_t display, cudaStream_t s) 
 }
 void launch_hash_build(const float4* pos, const float4* flux, uint32_t pw, uint32_t ph, uint32_t hash_num,
                        const float bbmin[3], float G, uint32_t flags, uint32_t* winner, uint32_t* count, cudaStream_t s) {
-    k_hash_clear<<<blocks_for(blocks_for(hash_num, 4), 256), 256, 0, s>>>(winner, count, hash_num);
+    k_hash_clear<<<blocks_for((hash_num - 1) / 4 + 1, 256), 256, 0, s>>>(winner, count, hash_num);
     const uint32_t n = pw * ph;
     if (n) k_hash_build<<<blocks_for(n, 256), 256, 0, s>>>(pos, flux, pw, ph, hash_num, bbmin[0], bbmin[1], bbmin[2], G, flags, winner, count);
 }
