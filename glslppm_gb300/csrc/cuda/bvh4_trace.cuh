@@ -31,25 +31,28 @@ __device__ __forceinline__ float slab_dir(float d) { return fabsf(d) < 1e-26f ? 
 
 // ---- conservative slab tests over the quantised boxes ------------------------------------------
 // A child plane is P = origin + q * 2^e (q a byte).  One byte permutation places the byte in the
-// mantissa of 1.0: f = 1 + q * 2^-15, and the plane's distance along the ray is
-//     fma(f, A, B - A -+ E),  A = 2^(e+15) * r (exact scaling of r = fl(1/d)),
+// mantissa of 0.5: f = 0.5 + q * 2^-16, and the plane's distance along the ray is
+//     fma(f, A, B - A/2 -+ E),  A = 2^(e+16) * r (exact scaling of r = fl(1/d)),
 //     B = fma(origin, r, n),  n = fl(-o * r),
 // the two planes of a child and axis in one two-lane operation (near with -E, far with +E): half the
 // instructions of q made a float of its own (permutation and subtraction) and two scalar fmas.
 // Against the exact distance (P' - o) / d to the enclosing plane P' = fl(origin + q 2^e) that the
-// builder checked, the roundings of r, n, B, B - A, -+ E, the fma and P' add at most
+// builder checked, the roundings of r, n, B, B - A/2, -+ E, the fma and P' add at most
 // 8 u S + 2^-8 * 2^e |r| (1 + O(u)), u = 2^-24, with S = (|origin| + |o| + 255 * 2^e) / |d| (each
-// rounding's error is u times a term bounded by S, and those of B - A and -+ E u times |A| more).
+// rounding's error is u times a term bounded by S, and those of B - A/2 and -+ E u times |A/2| more).
 // E = 16 u S' + 2^-7 * 2^e |r|, S' the same sum computed from |r|, |n| and |A| (relative error a few
 // u), exceeds that bound, so the near distance is never above the exact entry and the far distance
 // never below the exact exit: a box the exact arithmetic enters is never culled (Ize, "Robust BVH Ray
 // Traversal", JCGT 2013, applies the same argument to the plain slab test).  Where A overflows, the
-// distances become NaN, which the minimum and maximum drop: the box is entered.  The near plane of
-// each axis is chosen by the sign of the direction once per node, so a child needs no per-axis
-// min/max.
+// distances become NaN, which the minimum and maximum drop: the box is entered.  Where A does not,
+// |A/2| is at most half the largest float, so B - A/2 overflows only with |B| above that half, and a plane
+// is at most 0.0078 |A/2| from B: the infinite distance has the side that the plane is on.  (With the byte
+// under 1.0 and A half as large, B - A overflowed where B was next to nothing, and entered boxes were
+// culled.)  The near plane of each axis is chosen by the sign of the direction once per node, so a child
+// needs no per-axis min/max.
 constexpr float kSlabErr = 9.5367431640625e-07f;  // 16 * 2^-24
-// E's part in |A|: 255 * 2^-15 of S', and 2^-7 of a step (2^-22 of A)
-constexpr float kSlabErrA = 255.0f * kSlabErr / 32768.0f + 2.384185791015625e-07f;
+// E's part in |A|: 255 * 2^-16 of S', and 2^-7 of a step (2^-23 of A)
+constexpr float kSlabErrA = 255.0f * kSlabErr / 65536.0f + 1.1920928955078125e-07f;
 // a box entered later than the closest hit so far by less than this relative margin is still
 // visited: the exact triangle test's own rounding may put the winner's t just below its box entry
 constexpr float kCullMargin = 1.000244140625f;    // 1 + 2^-12
@@ -75,15 +78,15 @@ __device__ __forceinline__ void ray4_setup(Ray4& R, float ox, float oy, float oz
 
 // one axis of a node for one ray
 struct Slab4 {
-    unsigned long long A, B;  // A twice; B - A - E (near planes) and B - A + E (far planes)
+    unsigned long long A, B;  // A twice; B - A/2 - E (near planes) and B - A/2 + E (far planes)
     uint32_t near, far;       // words holding the near-plane and far-plane bytes of the four children
 };
 
 // e: the axis' exponent byte; lo, hi: the words of its lower and upper bytes
 __device__ __forceinline__ Slab4 slab4(uint32_t e, float origin, float lo, float hi, float r, float n) {
     Slab4 s;
-    const float A = (node_scale(e) * r) * 32768.0f;
-    const float C = fmaf(origin, r, n) - A;
+    const float A = (node_scale(e) * r) * 65536.0f;
+    const float C = fmaf(-0.5f, A, fmaf(origin, r, n));
     const float E = fmaf(kSlabErrA, fabsf(A), kSlabErr * fmaf(fabsf(origin), fabsf(r), fabsf(n)));
     s.A = pack2(A, A);
     s.B = pack2(C - E, C + E);
@@ -96,9 +99,9 @@ __device__ __forceinline__ Slab4 slab4(uint32_t e, float origin, float lo, float
 // near and far distance of child K along one axis
 template <int K>
 __device__ __forceinline__ void slab4_child(const Slab4& s, float& near, float& far) {
-    constexpr uint32_t sel = 0x7604u | ((uint32_t)K << 4);  // byte K under the exponent of 1.0
-    const float fn = __uint_as_float(__byte_perm(s.near, 0x3F800000u, sel));
-    const float ff = __uint_as_float(__byte_perm(s.far, 0x3F800000u, sel));
+    constexpr uint32_t sel = 0x7604u | ((uint32_t)K << 4);  // byte K under the exponent of 0.5
+    const float fn = __uint_as_float(__byte_perm(s.near, 0x3F000000u, sel));
+    const float ff = __uint_as_float(__byte_perm(s.far, 0x3F000000u, sel));
     unpack2(fma2(pack2(fn, ff), s.A, s.B), near, far);
 }
 
