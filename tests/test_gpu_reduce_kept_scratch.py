@@ -29,6 +29,11 @@ def used(cu):
     return n.value, torch.cuda.mem_get_info()[0]
 
 
+def no_more(before, now):
+    """(less is what an object of another test gives back when it is collected)"""
+    assert now[0] <= before[0] and now[1] >= before[1], (before, now)
+
+
 def reduce(ptr, want):
     from glslppm_gb300 import native as N
     out = (C.c_float * 4)()
@@ -65,7 +70,7 @@ def test_fresh_threads(driver):
     for _ in range(8):
         both()
     assert not bad, bad
-    assert used(driver) == before
+    no_more(before, used(driver))
 
 
 def test_two_contexts(driver):
@@ -90,7 +95,7 @@ def test_two_contexts(driver):
         before = used(driver)
         for _ in range(8):
             both()
-        assert used(driver) == before
+        no_more(before, used(driver))
     finally:
         driver.cuCtxDestroy_v2(second)
         assert driver.cuCtxSetCurrent(first) == 0
@@ -118,7 +123,7 @@ def test_contexts_that_come_and_go(driver):
     before = used(driver)
     for _ in range(6):
         one()
-    assert used(driver) == before
+    no_more(before, used(driver))
 
 
 def test_larger_sizes_replace_the_buffers(driver):
@@ -134,7 +139,7 @@ def test_larger_sizes_replace_the_buffers(driver):
     before = used(driver)
     for _ in range(4):
         sizes()
-    assert used(driver) == before
+    no_more(before, used(driver))
 
 
 def test_more_threads_than_buffers():
@@ -188,4 +193,4 @@ def test_a_capturing_stream_keeps_nothing(driver):
     before = used(driver)
     for _ in range(6):
         one()
-    assert used(driver) == before
+    no_more(before, used(driver))
