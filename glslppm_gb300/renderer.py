@@ -402,7 +402,8 @@ class Renderer:
         return float(ms.value)
 
     def set_tuning(self, tuning=None, **fields) -> None:
-        """Launch shapes (sppm_tuning): an N.Tuning, or its fields by name (others 0 = default)."""
+        """Launch shapes (sppm_tuning): an N.Tuning, or its fields by name (others 0: the default shape, and
+        binned rays).  To change one shape and keep the order of the rays, change it in get_tuning's report."""
         t = tuning if tuning is not None else N.Tuning(**fields)
         N.check(N.lib.sppm_set_tuning(self._h, C.byref(t)))
 
